@@ -295,6 +295,20 @@ int srf_emap_block_full(const float *crystal_table, int32_t n_blocks, int32_t m,
                         const int32_t grid[3], const float center[3], const float size[3],
                         void *stream);
 
+/* The same sum from the axial columns of the table (rows with the same x and y to the bit): the lines
+ * between two columns share their transaxial geometry and are accumulated in shared memory, each
+ * pair once for both orders. Several times faster for the crystal tables of cylindrical scanners;
+ * tables whose columns hold fewer than four rows on average go line by line as above. workspace:
+ * 8-byte aligned device memory of at least srf_emap_workspace() bytes, free again when the stream
+ * has passed the call; srf_emap_workspace() is 0 (and workspace may be NULL) for sizes that always
+ * go line by line (more than 2^20 rows, or more than 896 axial voxels). */
+int64_t srf_emap_workspace(int32_t n_blocks, int32_t m, const int32_t grid[3]);
+int srf_emap_block_full_ws(const float *crystal_table, int32_t n_blocks, int32_t m,
+                           float *emap, const int64_t emap_strides[3],
+                           float *emap_t, const int64_t emap_t_strides[3],
+                           const int32_t grid[3], const float center[3], const float size[3],
+                           void *workspace, int64_t workspace_bytes, void *stream);
+
 /* ------------------------------------------------------------------ single-scatter simulation */
 
 /* Raw single-scatter sums for crystal pairs (loop_all_lors / loop_all_s / get_scale of

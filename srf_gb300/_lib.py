@@ -27,7 +27,7 @@ EXPORTS = (
     "srf_last_error", "srf_version", "srf_set_group_lanes", "srf_set_tuning", "srf_projection", "srf_backprojection",
     "srf_projection_tof", "srf_backprojection_tof", "srf_projection_adjoint", "srf_fold_views",
     "srf_copy_view", "srf_count_pairs", "srf_projection_batch", "srf_projection_adjoint_batch", "srf_osem_subset", "srf_osem_update", "srf_osem_subset_batch",
-    "srf_osem_update_batch", "srf_emap_block_full", "srf_sss",
+    "srf_osem_update_batch", "srf_emap_block_full", "srf_emap_block_full_ws", "srf_emap_workspace", "srf_sss",
     "srf_backprojection_tof_noalloc", "srf_listmode_snap", "srf_lm2sino", "srf_attenuation",
     "srf_conv3d_fwd", "srf_conv3d_wgrad", "srf_conv3d_flip_weights", "srf_cnn_relu_bwd",
     "srf_set_conv_tc", "srf_conv_tc_status", "srf_conv_last_path",
@@ -65,6 +65,7 @@ def load(build_if_missing: bool = False):
         lib = ctypes.CDLL(path)
         lib.srf_last_error.restype = ctypes.c_char_p
         lib.srf_version.restype = ctypes.c_int
+        lib.srf_emap_workspace.restype = ctypes.c_int64
         for name in EXPORTS:
             getattr(lib, name)  # raises AttributeError if a symbol is missing
         _lib = lib

@@ -340,7 +340,8 @@ __device__ __forceinline__ void emap_warp(LeanRec *wrecs, const float *__restric
 
 template <int G, int U, int MINB, bool QDIV>
 __global__ void __launch_bounds__(kOsemBlock, MINB)
-k_emap_fused(const float *__restrict__ table, int nb, int m, Grid g, View v, View vt) {
+k_emap_fused(const float *__restrict__ table, int nb, int m, Grid g, View v, View vt, const int *__restrict__ done) {
+    if (done != nullptr && *done) return;  // the column form has the image
     __shared__ LeanRec recs[kOsemBlock / 32][32];
     const int wib = threadIdx.x >> 5;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -352,12 +353,13 @@ k_emap_fused(const float *__restrict__ table, int nb, int m, Grid g, View v, Vie
         emap_warp<G, U, QDIV>(recs[wib], table, nb, m, n, g, k, tp, v, vt, base);
 }
 
-int fused_emap(const float *table, int nb, int m, const Grid &g, const View &v, const View &vt, cudaStream_t s) {
+int fused_emap(const float *table, int nb, int m, const Grid &g, const View &v, const View &vt, const int *done,
+               cudaStream_t s) {
     const int64_t n = (int64_t)nb * nb * (int64_t)m * m;
     if (n == 0) return ok();
     auto kern = grid_qdiv(g) ? k_emap_fused<32, 4, 5, true> : k_emap_fused<32, 4, 5, false>;
     unsigned blocks = grid_for(kern, n, kOsemBlock, 0, kOsemBlock);
-    kern<<<blocks, kOsemBlock, 0, s>>>(table, nb, m, g, v, vt);
+    kern<<<blocks, kOsemBlock, 0, s>>>(table, nb, m, g, v, vt, done);
     return check_cuda("emap kernel launch");
 }
 
