@@ -301,8 +301,8 @@ int srf_emap_block_full(const float *crystal_table, int32_t n_blocks, int32_t m,
  * tables whose columns hold fewer than four rows on average go line by line as above. workspace:
  * 8-byte aligned device memory of at least srf_emap_workspace() bytes, free again when the stream
  * has passed the call; srf_emap_workspace() is 0 (and workspace may be NULL) for sizes that always
- * go line by line (more than 2^20 rows, or more than 896 axial voxels). */
-int64_t srf_emap_workspace(int32_t n_blocks, int32_t m, const int32_t grid[3]);
+ * go line by line (more than 2^20 rows). */
+int64_t srf_emap_workspace(int32_t n_blocks, int32_t m);
 int srf_emap_block_full_ws(const float *crystal_table, int32_t n_blocks, int32_t m,
                            float *emap, const int64_t emap_strides[3],
                            float *emap_t, const int64_t emap_t_strides[3],

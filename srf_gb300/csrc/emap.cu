@@ -28,7 +28,7 @@ struct EmapCols {
     int *off;                  // [rows + 1] first member of each column
     int *fill;                 // [rows]
     float2 *xy;                // [rows] (x, y) of each column
-    float *zu, *z;             // [rows] members' z, as collected and sorted by column
+    float *zu, *fz;            // [rows] members' z as collected, and their axial coordinates (voxels) sorted by column
     int *meta;                 // [0] number of columns, [1] 1: the column form runs
 };
 
@@ -51,7 +51,7 @@ static EmapCols emap_cols(int32_t *ws, int64_t rows) {
     c.off = ws; ws += rows + 1;
     c.fill = ws; ws += rows;
     c.zu = reinterpret_cast<float *>(ws); ws += rows;
-    c.z = reinterpret_cast<float *>(ws); ws += rows;
+    c.fz = reinterpret_cast<float *>(ws); ws += rows;
     c.meta = ws;
     return c;
 }
@@ -129,9 +129,10 @@ __global__ void k_cols_collect(const float *__restrict__ table, EmapCols c, int 
     }
 }
 
-// Each column's members by z, ascending (rank by counting; the order of equal values is free).
-__global__ void k_cols_sort(EmapCols c) {
+// Each column's members by z, ascending (rank by counting), as axial coordinates in voxels.
+__global__ void k_cols_sort(EmapCols c, Grid g) {
     if (!c.meta[1]) return;
+    const GridK k = make_gridk<false>(g, TofParams{0, 0, 0});
     const int cols = c.meta[0];
     for (int col = blockIdx.x; col < cols; col += gridDim.x) {
         const int lo = c.off[col], n = c.off[col + 1] - lo;
@@ -142,87 +143,145 @@ __global__ void k_cols_sort(EmapCols c) {
                 const float v = c.zu[lo + j];
                 rank += (v < z || (v == z && j < i)) ? 1 : 0;
             }
-            c.z[lo + rank] = z;
+            c.fz[lo + rank] = __fdiv_rn(__fdiv_rn(__fsub_rn(z, g.cz), k.dx_), k.dz) + k.nz2;
         }
     }
 }
 
 // ---------------------------------------------------------------- lines between two columns
 constexpr int kParams = 64;  // members of the second column whose line constants are held at a time
+constexpr int kWindow = 56;  // axial voxels of a lane's cells
 
-// The lines from one member (axial face coordinate zA) to `cnt` members of the other column, on one
-// slab per lane. prm[j] = (D, wc, 1 / |axial step per slab|): D the axial extent in voxels, wc the
-// weight of a whole slab. ta, tb: the slab's two faces along the line (0 at zA, 1 at the other end),
-// the one with the lower axial coordinate first. fq: fraction of the slab before its in-plane
-// crossing. Cell (a, c): lane's word at s[(c + row) * 32], rows from row a of the two in-plane cells.
-// Slots and weights as lean_slab's; RANGE adds its axial range tests (the in-plane ones are per
-// slab and decided when the cells are written out).
-template <bool RANGE>
-__device__ __forceinline__ void column_lines(float *s, const float4 *prm, int j0, int cnt, float zA, float ta, float tb,
-                                             float fq, int nz) {
-    const unsigned cA = 0u - (unsigned)kFloorBits * 32u, cB = cA + (unsigned)nz * 32u;
-    constexpr int K = 4;  // lines whose arithmetic is interleaved before their additions run in order
-    for (int j = j0; j < cnt; j += K) {
-        unsigned i0[K], i1[K], i2[K];
-        float w0[K], w1[K], w2[K];
+// Line constants: D the axial extent in voxels, wc the weight of a whole slab, iz = 1 / |axial step per
+// slab|, nwc = -wc. Lines that rise and lines that fall with the slab's first face are two runs; a
+// run of cnt lines, ascending in D, is dealt to groups of four, line j to place 4 (j mod q) + j / q,
+// q = cnt / 4, so that a group's lines end a quarter of the run apart; the last cnt mod 4 lines form
+// a group of their own, padded with lines of weight 0.
+struct LineParams {
+    float D[kParams + 8], wc[kParams + 8], iz[kParams + 8], nwc[kParams + 8];
+};
+
+// The lines of one run (groups of four from place g0) from one member (axial face coordinate zA,
+// relative to the lane's window), on one slab per lane. ta, tb: the slab's two faces along the line (0
+// at zA, 1 at the other end), the one with the lower axial coordinate first. fq: fraction of the slab
+// before its in-plane crossing. Cells: the lane's words s[c * 32] of the first in-plane cell and
+// s[(kWindow + c) * 32] of the second. Slots and weights as lean_slab's, without its range tests:
+// every voxel lies in the window, and what lies outside the image is not written out.
+__device__ __forceinline__ void column_lines(float *s, const LineParams &prm, int g0, int groups, float zA, float ta,
+                                             float tb, float fq) {
+    constexpr unsigned cA = 0u - (unsigned)kFloorBits * 32u, dB = (unsigned)kWindow * 32u;
+    const float2 one_m = make_float2(-1.0f, -1.0f), magic = make_float2(kFloorMagic, kFloorMagic);
+    const float2 magic_m = make_float2(-kFloorMagic, -kFloorMagic);
+    const float2 zA2 = make_float2(zA, zA), ta2 = make_float2(ta, ta), tb2 = make_float2(tb, tb), fq2 = make_float2(fq, fq);
+    for (int g = 0; g < groups; ++g) {
+        const int at = g0 + 4 * g;
+        const float4 D4 = *reinterpret_cast<const float4 *>(prm.D + at), wc4 = *reinterpret_cast<const float4 *>(prm.wc + at);
+        const float4 iz4 = *reinterpret_cast<const float4 *>(prm.iz + at), nw4 = *reinterpret_cast<const float4 *>(prm.nwc + at);
+        const float2 D_[2] = {{D4.x, D4.y}, {D4.z, D4.w}}, wc_[2] = {{wc4.x, wc4.y}, {wc4.z, wc4.w}};
+        const float2 iz_[2] = {{iz4.x, iz4.y}, {iz4.z, iz4.w}}, nw_[2] = {{nw4.x, nw4.y}, {nw4.z, nw4.w}};
+        unsigned i0[4], i1[4], i2[4];
+        float w0[4], w1[4], w2[4];
+        int b1[4], b2[4];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const float4 p = prm[min(j + k, cnt - 1)];
-            const float wc = j + k < cnt ? p.y : 0.0f;
-            float z1 = fmaf(p.x, ta, zA), z2 = fmaf(p.x, tb, zA);
-            if (RANGE) {
-                z1 = fminf(fmaxf(z1, -2097152.0f), 2097152.0f);
-                z2 = fminf(fmaxf(z2, -2097152.0f), 2097152.0f);
-            }
-            const float f1 = __fadd_rd(z1, kFloorMagic), f2 = __fadd_rd(z2, kFloorMagic);
-            const unsigned b1 = (unsigned)__float_as_int(f1), b2 = (unsigned)__float_as_int(f2);
-            const float fz = b1 != b2 ? ((f2 - kFloorMagic) - z1) * p.z : 1.0f;
-            const bool qfirst = fq > fz;
-            w0[k] = fminf(fq, fz) * wc;
-            w1[k] = fabsf(fq - fz) * wc;
-            w2[k] = fmaf(-fmaxf(fq, fz), wc, wc);
-            i0[k] = b1 * 32u + cA;
-            i1[k] = (qfirst ? b2 : b1) * 32u + (qfirst ? cA : cB);
-            i2[k] = b2 * 32u + cB;
-            if (RANGE) {
-                const int c1 = (int)b1 - kFloorBits, c2 = (int)b2 - kFloorBits;
-                const bool B = (unsigned)c1 < (unsigned)nz, D = (unsigned)c2 < (unsigned)nz && c1 >= -1;
-                const bool v1 = qfirst ? D : B;
-                w0[k] = B ? w0[k] : 0.0f; i0[k] = B ? i0[k] : 0u;
-                w1[k] = v1 ? w1[k] : 0.0f; i1[k] = v1 ? i1[k] : (unsigned)nz * 32u;
-                w2[k] = D ? w2[k] : 0.0f; i2[k] = D ? i2[k] : 0u;
-            }
+        for (int h = 0; h < 2; ++h) {  // two lines at a time in packed FP32 arithmetic
+            const float2 z1 = __ffma2_rn(D_[h], ta2, zA2), z2 = __ffma2_rn(D_[h], tb2, zA2);
+            const float2 f1 = __fadd2_rd(z1, magic), f2 = __fadd2_rd(z2, magic);
+            const float2 fr = __fmul2_rn(__ffma2_rn(z1, one_m, __fadd2_rn(f2, magic_m)), iz_[h]);
+            b1[2 * h] = __float_as_int(f1.x); b1[2 * h + 1] = __float_as_int(f1.y);
+            b2[2 * h] = __float_as_int(f2.x); b2[2 * h + 1] = __float_as_int(f2.y);
+            const float2 fz = make_float2(f1.x != f2.x ? fr.x : 1.0f, f1.y != f2.y ? fr.y : 1.0f);
+            const float2 a0 = __fmul2_rn(make_float2(fminf(fq, fz.x), fminf(fq, fz.y)), wc_[h]);
+            const float2 a1 = __fmul2_rn(__ffma2_rn(fz, one_m, fq2), wc_[h]);  // > 0: the in-plane crossing is later
+            const float2 a2 = __ffma2_rn(make_float2(fmaxf(fq, fz.x), fmaxf(fq, fz.y)), nw_[h], wc_[h]);
+            w0[2 * h] = a0.x; w0[2 * h + 1] = a0.y;
+            w1[2 * h] = a1.x; w1[2 * h + 1] = a1.y;
+            w2[2 * h] = a2.x; w2[2 * h + 1] = a2.y;
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (RANGE) {  // dropped slots add zero to some cell, so the additions keep their order
-                s[i0[k]] += w0[k];
-                s[i1[k]] += w1[k];
-                s[i2[k]] += w2[k];
-                continue;
+        for (int k = 0; k < 4; ++k) {
+            i0[k] = (unsigned)b1[k] * 32u + cA;
+            i2[k] = (unsigned)b2[k] * 32u + (cA + dB);
+            i1[k] = w1[k] > 0.0f ? i2[k] - dB : i0[k] + dB;
+        }
+        // A line's slots 0 and 1 are different cells, and slot 2 (both coordinates cross) a third. When
+        // the group's lines use different voxels too, their additions overlap; else they run in order.
+        if (__all_sync(0xffffffffu, b1[1] > b2[0] && b1[2] > b2[1] && b1[3] > b2[2])) {
+            float a[4], b[4], c[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                a[k] = s[i0[k]];
+                b[k] = s[i1[k]];
+                c[k] = w2[k] != 0.0f ? s[i2[k]] : 0.0f;
             }
-            // slots 0 and 1 are different cells, and slot 2 (both coordinates cross) a third
-            const float a = s[i0[k]], b = s[i1[k]];
-            if (w2[k] != 0.0f) s[i2[k]] += w2[k];
-            s[i0[k]] = a + w0[k];
-            s[i1[k]] = b + w1[k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s[i0[k]] = a[k] + w0[k];
+                s[i1[k]] = b[k] + fabsf(w1[k]);
+                if (w2[k] != 0.0f) s[i2[k]] = c[k] + w2[k];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float a = s[i0[k]], b = s[i1[k]];
+                if (w2[k] != 0.0f) s[i2[k]] += w2[k];
+                s[i0[k]] = a + w0[k];
+                s[i1[k]] = b + fabsf(w1[k]);
+            }
         }
     }
 }
 
-// One warp (= one block) takes one pair of columns A < B and one tile of 32 slabs; each lane owns a
-// slab: two in-plane cells (before and after its crossing) of nz voxels each in shared memory, private
-// to the lane, so the c1 c2 lines accumulate there without atomics. The cells then go to the image
-// with one reduction per voxel, times two: the line from B to A is the line from A to B, and both
-// are in the sum (a column with itself has no transaxial extent and is skipped by the short-LOR rule).
-// Bound: instruction issue of the loop over the lines, ~32 instructions per line and 32 slabs against
-// ~120 of the line-by-line form and half the lines; shared memory (2 nz words per lane, 28 KB at
-// nz = 109) allows 7 warps per SM, whose additions' latency the K = 4 interleaving covers.
-// Measured, 32,448 crystals (624 columns of 52) on 200 x 200 x 109: 121.6 ms against 308 ms line by line.
+// The same lines straight into the image (imA, imB: the slab's two in-plane cells, null outside the
+// image), with every range test: steep lines, and slabs beyond the columns.
+__device__ __forceinline__ void column_lines_direct(const LineParams &prm, int g0, int groups, float zA, float ta, float tb,
+                                                    float fq, int nz, int64_t st_z, float *imA, float *imB) {
+    for (int j = g0; j < g0 + 4 * groups; ++j) {
+        const float D = prm.D[j], wc = 2.0f * prm.wc[j];
+        if (wc == 0.0f) continue;
+        const float z1 = fminf(fmaxf(fmaf(D, ta, zA), -2097152.0f), 2097152.0f);
+        const float z2 = fminf(fmaxf(fmaf(D, tb, zA), -2097152.0f), 2097152.0f);
+        const float f1 = __fadd_rd(z1, kFloorMagic), f2 = __fadd_rd(z2, kFloorMagic);
+        const int c1 = __float_as_int(f1) - kFloorBits, c2 = __float_as_int(f2) - kFloorBits;
+        const float fz = c1 != c2 ? ((f2 - kFloorMagic) - z1) * prm.iz[j] : 1.0f;
+        const bool qfirst = fq > fz;
+        const bool B = (unsigned)c1 < (unsigned)nz, C = (unsigned)c2 < (unsigned)nz && c1 >= -1;
+        const float w0 = fminf(fq, fz) * wc, w1 = fabsf(fq - fz) * wc, w2 = fmaf(-fmaxf(fq, fz), wc, wc);
+        if (imA && B && w0 != 0.0f) atomicAdd(imA + c1 * st_z, w0);
+        if (imA && qfirst && C && w1 != 0.0f) atomicAdd(imA + c2 * st_z, w1);
+        if (imB && !qfirst && B && w1 != 0.0f) atomicAdd(imB + c1 * st_z, w1);
+        if (imB && C && w2 != 0.0f) atomicAdd(imB + c2 * st_z, w2);
+    }
+}
+
+// Last member (exclusive) of the piece that starts at member i: at most kParams members within `ext`
+// axial voxels of it (z ascending).
+__device__ __forceinline__ int piece_end(const float *fz, int i, int n, float ext, int lane) {
+    const float z0 = fz[i];
+    int e = i;
+#pragma unroll
+    for (int r = 0; r < kParams / 32; ++r) {
+        const int j = i + lane + 32 * r;
+        e += __popc(__ballot_sync(0xffffffffu, j < n && fz[min(j, n - 1)] - z0 <= ext));
+    }
+    return max(e, i + 1);
+}
+
+// One warp (= one block) takes one pair of columns A < B and one tile of 32 slabs, and of each column
+// a piece at a time (at most kWindow - 4 voxels long). A line between two points lies between the
+// lines through the pieces' ends, so on any slab the pieces' lines use at most kWindow voxels along
+// the axis, from a first voxel of the slab's own: each lane owns a slab and holds its two in-plane
+// cells (before and after the crossing) over that window in shared memory. The lines accumulate there
+// without atomics, then the cells go to the image with one reduction per voxel, times two: the line
+// from B to A is the line from A to B, and both are in the sum (a column with itself has no
+// transaxial extent and is skipped by the short-LOR rule).
+// Bound: instruction issue of column_lines, ~35 instructions per line and 32 slabs against ~120 of the
+// line-by-line form, and half the lines. The window sets the warps an SM can hold: whole columns of
+// cells (109 voxels: 28 KB a warp, 7 warps) ran at 51 % of the issue slots, 115 ms; kWindow 56 (14 KB,
+// 13 warps) at 66 %, 85 ms, all on 32,448 crystals (624 columns of 52) and 200 x 200 x 109; line by line 308 ms.
 __global__ void __launch_bounds__(32)
 k_emap_columns(EmapCols c, Grid g, View v, View vt, int tiles) {
-    extern __shared__ float s_cells[];                      // [2 nz][32]
-    __shared__ float4 prm[kParams];
+    __shared__ float s_cells[2 * kWindow * 32];
+    __shared__ __align__(16) LineParams prm;
     if (!c.meta[1]) return;
     const int lane = threadIdx.x;
     const int cols = c.meta[0];
@@ -231,7 +290,7 @@ k_emap_columns(EmapCols c, Grid g, View v, View vt, int tiles) {
     const GridK k = make_gridk<false>(g, tp);
     const int nz = g.nz;
     float *s = s_cells + lane;
-    for (int r = 0; r < 2 * nz; ++r) s[r * 32] = 0.0f;
+    for (int r = 0; r < 2 * kWindow; ++r) s[r * 32] = 0.0f;
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
         const int64_t pair = it / tiles;
         // pair = B (B - 1) / 2 + A, A < B
@@ -268,66 +327,108 @@ k_emap_columns(EmapCols c, Grid g, View v, View vt, int tiles) {
         const bool okA = act && 0 <= cq1 && cq1 < nq, okB = act && 0 <= cq2 && cq2 < nq && cq1 >= -1;
         if (!__any_sync(0xffffffffu, okA || okB)) continue;
         const float t_lo = __fdiv_rn(__fsub_rn(pp1, p1), pd), t_hi = __fdiv_rn(__fsub_rn(pp2, p1), pd);
-        const int a0 = c.off[A], na = c.off[A + 1] - a0, b0 = c.off[B], nb = c.off[B + 1] - b0;
-        auto face_z = [&](float z) { return __fdiv_rn(__fdiv_rn(__fsub_rn(z, g.cz), k.dx_), k.dz) + k.nz2; };
-        // members are sorted: inside the box by a margin when the first and the last of both columns are
-        // (and the slab lies between the columns, so that every axial coordinate does too)
-        const float zlo = fminf(face_z(c.z[a0]), face_z(c.z[b0])), zhi = fmaxf(face_z(c.z[a0 + na - 1]), face_z(c.z[b0 + nb - 1]));
         const bool between = __all_sync(0xffffffffu, t_lo >= 0.0f && t_lo <= 1.0f && t_hi >= 0.0f && t_hi <= 1.0f);
-        const bool inside = between && zlo >= kInteriorMargin && zhi <= (float)nz - kInteriorMargin;
+        const int a0 = c.off[A], na = c.off[A + 1] - a0, b0 = c.off[B], nb = c.off[B + 1] - b0;
+        const float *zA_ = c.fz + a0, *zB_ = c.fz + b0;
+        // pieces of equal length, as few as fit
+        const float extA = zA_[na - 1] - zA_[0], extB = zB_[nb - 1] - zB_[0];
+        const float lenA = extA / fmaxf(ceilf(extA / (kWindow - 5.0f)), 1.0f) + 0.5f;
+        const float lenB = extB / fmaxf(ceilf(extB / (kWindow - 5.0f)), 1.0f) + 0.5f;
         const float ku = 1.0f + kq * kq, ipd = 1.0f / pd;
-        for (int jb = 0; jb < nb; jb += kParams) {
-            const int cnt = min(kParams, nb - jb);
-            for (int ia = 0; ia < na; ++ia) {
-                const float zA = face_z(__ldg(c.z + a0 + ia));
-                __syncwarp();
-                int down = 0;  // members below A's: D < 0 (they come first)
-                for (int j = lane; j < kParams; j += 32) {
-                    float D = 0.0f, wc = 0.0f, iz = 0.0f;
-                    if (j < cnt) {
-                        D = face_z(__ldg(c.z + b0 + jb + j)) - zA;
-                        const float kz = D * k.dz * ipd;
-                        wc = isfinite(D) ? sqrtf(ku + kz * kz) * k.dx_ : 0.0f;
-                        D = isfinite(D) ? D : 0.0f;
-                        iz = fabsf(pd) / fabsf(D);
-                    }
-                    prm[j] = make_float4(D, wc, iz, 0.0f);
-                    down += __popc(__ballot_sync(0xffffffffu, D < 0.0f));
-                }
-                __syncwarp();
-                // the face with the lower axial coordinate: the lower slab face when the line rises with p
-                const bool up = pd > 0.0f;
-                if (inside) {
-                    column_lines<false>(s, prm, 0, down, zA, up ? t_hi : t_lo, up ? t_lo : t_hi, fq, nz);
-                    column_lines<false>(s, prm, down, cnt, zA, up ? t_lo : t_hi, up ? t_hi : t_lo, fq, nz);
-                } else {
-                    column_lines<true>(s, prm, 0, down, zA, up ? t_hi : t_lo, up ? t_lo : t_hi, fq, nz);
-                    column_lines<true>(s, prm, down, cnt, zA, up ? t_lo : t_hi, up ? t_hi : t_lo, fq, nz);
-                }
-            }
-        }
-        // the cells into the image, and back to zero
+        const bool up = pd > 0.0f;  // a line with D > 0 has its lower axial coordinate at the slab's lower face
+        // views: cells (ip, cq1) and (ip, cq2)
         const bool tview = !xdom && vt.ptr != nullptr;
         const int64_t st_p = tview ? vt.st[1] : (xdom ? v.st[0] : v.st[1]);
         const int64_t st_q = tview ? vt.st[0] : (xdom ? v.st[1] : v.st[0]);
         const int64_t st_z = tview ? vt.st[2] : v.st[2];
         float *im = tview ? vt.ptr : v.ptr;
-        float *imA = im + ip * st_p + (int64_t)(okA ? cq1 : 0) * st_q, *imB = im + ip * st_p + (int64_t)(okB ? cq2 : 0) * st_q;
-        for (int r = 0; r < nz; ++r) {
-            const float a = s[r * 32], b = s[(nz + r) * 32];
-            s[r * 32] = 0.0f;
-            s[(nz + r) * 32] = 0.0f;
-            if (okA && a != 0.0f) atomicAdd(imA + r * st_z, 2.0f * a);
-            if (okB && b != 0.0f) atomicAdd(imB + r * st_z, 2.0f * b);
+        float *imA = okA ? im + ip * st_p + (int64_t)cq1 * st_q : nullptr, *imB = okB ? im + ip * st_p + (int64_t)cq2 * st_q : nullptr;
+        for (int ja = 0, ea; ja < na; ja = ea) {
+            ea = piece_end(zA_, ja, na, lenA, lane);
+            for (int jb = 0, eb; jb < nb; jb = eb) {
+                eb = piece_end(zB_, jb, nb, lenB, lane);
+                const int cnt = eb - jb;
+                // the window's first voxel, and whether the window holds the pieces' lines: slabs between the
+                // columns, at most one voxel of axial step per slab
+                const float zA0 = zA_[ja], zB0 = zB_[jb], zA1 = zA_[ea - 1], zB1 = zB_[eb - 1];
+                const float m = fminf(fmaf(zB0 - zA0, t_lo, zA0), fmaf(zB0 - zA0, t_hi, zA0));
+                // (coordinates and extents below 2^13 keep their rounding far below the margin of 0.01)
+                const float rise = fmaxf(fabsf(zB1 - zA0), fabsf(zB0 - zA1));
+                const float base = floorf(m - 0.01f);
+                const bool fast = between && __all_sync(0xffffffffu, rise * fabsf(ipd) <= 1.0f && rise < 8192.0f && fabsf(base) < 8192.0f);
+                for (int ia = ja; ia < ea; ++ia) {
+                    const float zA = zA_[ia];
+                    __syncwarp();
+                    // constants of the lines to this lane's members; falling lines (D < 0) come first
+                    float D[kParams / 32], wc[kParams / 32];
+                    int n_down = 0;
+#pragma unroll
+                    for (int r = 0; r < kParams / 32; ++r) {
+                        const int j = lane + 32 * r;
+                        D[r] = wc[r] = 0.0f;
+                        if (j < cnt) {
+                            const float d = zB_[jb + j] - zA;
+                            const float kz = d * k.dz * ipd;
+                            if (isfinite(d)) { D[r] = d; wc[r] = sqrtf(ku + kz * kz) * k.dx_; }
+                        }
+                        n_down += __popc(__ballot_sync(0xffffffffu, D[r] < 0.0f));
+                    }
+                    const int n_up = cnt - n_down, g_down = (n_down + 3) >> 2, g_up = (n_up + 3) >> 2;
+#pragma unroll
+                    for (int r = 0; r < kParams / 32; ++r) {
+                        const int j = lane + 32 * r;
+                        if (j < cnt) {
+                            const bool first_run = j < n_down;
+                            const int i = first_run ? j : j - n_down, q = (first_run ? n_down : n_up) >> 2;
+                            const int quarter = (i >= q) + (i >= 2 * q) + (i >= 3 * q);
+                            const int at = (first_run ? 0 : 4 * g_down) + (i < 4 * q ? 4 * (i - quarter * q) + quarter : i);
+                            prm.D[at] = D[r];
+                            prm.wc[at] = wc[r];
+                            prm.nwc[at] = -wc[r];
+                            prm.iz[at] = fabsf(pd) / fabsf(D[r]);
+                        }
+                    }
+                    __syncwarp();
+                    if (lane < 8) {  // the padding of both runs' last groups: the run's last line, weightless
+                        const int n_run = lane < 4 ? n_down : n_up, rem = n_run & 3, run = lane < 4 ? 0 : 4 * g_down;
+                        const int at = run + (n_run & ~3) + (lane & 3);
+                        if (rem != 0 && (lane & 3) >= rem) {
+                            prm.D[at] = prm.D[run + n_run - 1];
+                            prm.wc[at] = prm.nwc[at] = prm.iz[at] = 0.0f;
+                        }
+                    }
+                    __syncwarp();
+                    const float t_dn = up ? t_hi : t_lo, t_up = up ? t_lo : t_hi;
+                    if (fast) {
+                        column_lines(s, prm, 0, g_down, zA - base, t_dn, t_up, fq);
+                        column_lines(s, prm, 4 * g_down, g_up, zA - base, t_up, t_dn, fq);
+                    } else {
+                        column_lines_direct(prm, 0, g_down, zA, t_dn, t_up, fq, nz, st_z, imA, imB);
+                        column_lines_direct(prm, 4 * g_down, g_up, zA, t_up, t_dn, fq, nz, st_z, imA, imB);
+                    }
+                }
+                if (!fast) continue;
+                // the cells into the image, and back to zero
+                const int z0 = (int)base;
+#pragma unroll 4
+                for (int r = 0; r < kWindow; ++r) {
+                    const float a = s[r * 32], b = s[(kWindow + r) * 32];
+                    s[r * 32] = 0.0f;
+                    s[(kWindow + r) * 32] = 0.0f;
+                    const int z = z0 + r;
+                    if ((unsigned)z >= (unsigned)nz) continue;
+                    if (imA && a != 0.0f) atomicAdd(imA + z * st_z, 2.0f * a);
+                    if (imB && b != 0.0f) atomicAdd(imB + z * st_z, 2.0f * b);
+                }
+            }
         }
     }
 }
 
 // Columns shorter than this on average go line by line: a column pair costs a tile ~1,300 instructions
-// to write its cells out, as much as ~11 lines of the line-by-line form.
+// to set up and to write its cells out, as much as ~11 lines of the line-by-line form.
 constexpr int kMinMembers = 4;
 constexpr int64_t kMaxRows = 1 << 20;
-constexpr int kMaxCellBytes = 224 * 1024;
 
 static int emap_args(const float *table, int32_t n_blocks, int32_t m, float *emap, const int64_t st[3], float *emap_t,
                      const int64_t st_t[3], const int32_t grid[3], const float center[3], const float size[3], Grid &g,
@@ -353,9 +454,9 @@ extern "C" int srf_emap_block_full(const float *crystal_table, int32_t n_blocks,
     return fused_emap(crystal_table, n_blocks, m, g, v, vt, nullptr, (cudaStream_t)stream);
 }
 
-extern "C" int64_t srf_emap_workspace(int32_t n_blocks, int32_t m, const int32_t grid[3]) {
+extern "C" int64_t srf_emap_workspace(int32_t n_blocks, int32_t m) {
     const int64_t rows = (int64_t)(n_blocks > 0 ? n_blocks : 0) * (m > 0 ? m : 0);
-    if (rows < 1 || rows > kMaxRows || !grid || (int64_t)grid[2] * 256 > kMaxCellBytes) return 0;
+    if (rows < 1 || rows > kMaxRows) return 0;
     return emap_words(rows) * 4;
 }
 
@@ -366,7 +467,7 @@ extern "C" int srf_emap_block_full_ws(const float *crystal_table, int32_t n_bloc
     Grid g; View v, vt; int rc;
     if ((rc = emap_args(crystal_table, n_blocks, m, emap, emap_strides, emap_t, emap_t_strides, grid, center, size, g, v, vt))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const int64_t need = srf_emap_workspace(n_blocks, m, grid);
+    const int64_t need = srf_emap_workspace(n_blocks, m);
     if (need == 0) return fused_emap(crystal_table, n_blocks, m, g, v, vt, nullptr, s);  // a size the columns do not serve
     if (!workspace) return fail(SRF_EINVAL, "workspace must not be NULL");
     if ((uintptr_t)workspace & 7) return fail(SRF_EINVAL, "workspace must be 8-byte aligned");
@@ -377,14 +478,12 @@ extern "C" int srf_emap_block_full_ws(const float *crystal_table, int32_t n_bloc
     k_cols_insert<<<grid_for(k_cols_insert, rows, 256), 256, 0, s>>>(crystal_table, c, slots, rows);
     k_cols_offsets<<<1, 1024, 0, s>>>(c, slots, rows, kMinMembers);
     k_cols_collect<<<grid_for(k_cols_collect, rows, 256), 256, 0, s>>>(crystal_table, c, rows);
-    k_cols_sort<<<grid_for(k_cols_sort, rows, 1, 0, 64), 64, 0, s>>>(c);
+    k_cols_sort<<<grid_for(k_cols_sort, rows, 1, 0, 64), 64, 0, s>>>(c, g);
     if ((rc = check_cuda("emap column launches"))) return rc;
-    const int smem = g.nz * 256;
-    if (smem > 32 * 1024) cudaFuncSetAttribute(k_emap_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int tiles = ((g.nx > g.ny ? g.nx : g.ny) + 31) / 32;
     // at most rows (rows - 1) / 2 column pairs; the kernel reads how many there are
     const int64_t items = (int64_t)rows * (rows - 1) / 2 * tiles;
-    k_emap_columns<<<grid_for(k_emap_columns, items, 1, smem, 32), 32, smem, s>>>(c, g, v, vt, tiles);
+    k_emap_columns<<<grid_for(k_emap_columns, items, 1, 0, 32), 32, 0, s>>>(c, g, v, vt, tiles);
     if ((rc = check_cuda("emap column kernel launch"))) return rc;
     return fused_emap(crystal_table, n_blocks, m, g, v, vt, c.meta + 1, s);
 }

@@ -241,7 +241,7 @@ def emap_block_full(table: torch.Tensor, n_blocks: int, shape, center, size) -> 
     m = table.shape[0] // n_blocks
     acc = new_xfast(shape, table.device)
     acc_t = new_yfast(shape, table.device)
-    need = int(_lib.load().srf_emap_workspace(i32(n_blocks), i32(m), i32x3(shape)))
+    need = int(_lib.load().srf_emap_workspace(i32(n_blocks), i32(m)))
     ws = torch.empty(need, dtype=torch.uint8, device=table.device) if need else None
     call("srf_emap_block_full_ws", ptr(table), i32(n_blocks), i32(m), ptr(acc), i64x3(acc.stride()),
          ptr(acc_t), i64x3(acc_t.stride()), i32x3(shape), f32x3(center), f32x3(size), ptr(ws), i64(need),
