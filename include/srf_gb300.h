@@ -144,6 +144,29 @@ int srf_projection_adjoint_batch(const float *lors, int64_t n, int32_t lor_strid
                                  float *images_t, const int64_t image_t_strides[3], const int32_t grid[3],
                                  const float center[3], const float size[3], void *stream);
 
+/* The batched pair on interleaved images: `width` (2, 4 or 8) values per voxel, image b < n_images
+ * <= width in place b, voxels x-fastest in il and y-fastest in the optional il_t (which then holds the
+ * y-dominant LORs' part). Same visits and weights as the forms above, several times fewer memory
+ * accesses. srf_interleave fills il (and il_t) from n_images images of any strides, zeros in the
+ * unused places; srf_deinterleave writes il (+ il_t) back. Interleaved images are aligned to
+ * 4 * width bytes. The adjoint adds to il and il_t. */
+int srf_interleave(const float *images, int64_t batch_stride, const int64_t image_strides[3],
+                   int32_t n_images, int32_t width, const int32_t grid[3], float *il, float *il_t,
+                   void *stream);
+int srf_deinterleave(const float *il, const float *il_t, int32_t n_images, int32_t width,
+                     const int32_t grid[3], float *images, int64_t batch_stride,
+                     const int64_t image_strides[3], void *stream);
+int srf_projection_il(const float *lors, int64_t n, int32_t lor_stride, const float *tof,
+                      int32_t tof_stride, float tof_bin, float tof_sigma2, float tof_nsigma,
+                      int32_t n_images, int32_t width, const float *il, const float *il_t,
+                      const int32_t grid[3], const float center[3], const float size[3], float *out,
+                      int64_t out_stride, void *stream);
+int srf_projection_adjoint_il(const float *lors, int64_t n, int32_t lor_stride, const float *tof,
+                              int32_t tof_stride, float tof_bin, float tof_sigma2, float tof_nsigma,
+                              int32_t n_images, int32_t width, const float *values, int64_t values_stride,
+                              float *il, float *il_t, const int32_t grid[3], const float center[3],
+                              const float size[3], void *stream);
+
 /* *count += number of (LOR, voxel) weight visits the projector (rules 0) or backprojector
  * (rules 1) rule set makes for these LORs (tof == NULL: non-TOF rules). `count` is a device
  * unsigned 64-bit counter. These are the "LOR-voxel updates" of the throughput metric; the CPU

@@ -7,8 +7,8 @@ projector (projector skip rules and 1/L^2 weights). The reference's backprojecto
 adjoint (no endpoint/steep skips, no 1/L^2), so it cannot serve as a gradient.
 
 ``image`` is (nx, ny, nz) or a batch (B, nx, ny, nz) of float32 CUDA tensors; the result is (N,)
-or (B, N). A batch runs through srf_projection_batch / srf_projection_adjoint_batch, which set up
-and traverse each LOR once for up to 8 images. ``poisson_nll(p, y)`` is the list-mode/binned Poisson negative log-likelihood
+or (B, N). A batch runs through srf_projection_il / srf_projection_adjoint_il, which set up and
+traverse each LOR once for up to 8 images interleaved by voxel. ``poisson_nll(p, y)`` is the list-mode/binned Poisson negative log-likelihood
 sum(p - y log p) used as the training loss.
 """
 from __future__ import annotations
@@ -20,6 +20,10 @@ import torch
 from . import kernels
 
 
+def _joined(parts):
+    return parts[0] if len(parts) == 1 else torch.cat(parts)
+
+
 class _Project(torch.autograd.Function):
     @staticmethod
     def forward(ctx, image: torch.Tensor, lors: torch.Tensor, center, size, tof, tof_nsigma):
@@ -28,8 +32,8 @@ class _Project(torch.autograd.Function):
         if image.dim() == 3:
             return kernels.project(lors, image.detach(), center, size, tof=tof, tof_nsigma=tof_nsigma)
         B = kernels.MAX_BATCH
-        return torch.cat([kernels.project_batch(lors, image[k:k + B].detach(), center, size, tof=tof,
-                                                tof_nsigma=tof_nsigma) for k in range(0, image.shape[0], B)])
+        return _joined([kernels.project_batch(lors, image[k:k + B].detach(), center, size, tof=tof,
+                                              tof_nsigma=tof_nsigma) for k in range(0, image.shape[0], B)])
 
     @staticmethod
     def backward(ctx, grad_p: torch.Tensor):
@@ -42,8 +46,8 @@ class _Project(torch.autograd.Function):
                                        tof_nsigma=tof_nsigma, adjoint=True)
         else:
             B = kernels.MAX_BATCH
-            grad = torch.cat([kernels.adjoint_batch(lors, g[k:k + B], shape, center, size, tof=tof,
-                                                    tof_nsigma=tof_nsigma) for k in range(0, g.shape[0], B)])
+            grad = _joined([kernels.adjoint_batch(lors, g[k:k + B], shape, center, size, tof=tof,
+                                                  tof_nsigma=tof_nsigma) for k in range(0, g.shape[0], B)])
         return grad, None, None, None, None, None
 
 

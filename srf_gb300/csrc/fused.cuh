@@ -185,6 +185,13 @@ __device__ __forceinline__ LorRec setup_rec(const float *l, float tv, float yv, 
     return R;
 }
 
+// The x-dominant in-plane coordinate is divided by dy = (sy / ny) / (sx / nx) in the reference;
+// dy == 1 (square transaxial voxels) makes that division an identity the kernels compile out.
+inline bool grid_qdiv(const Grid &g) {
+    const float dx_ = g.sx / (float)g.nx;
+    return (g.sy / (float)g.ny) / dx_ != 1.0f;
+}
+
 // The standalone projector / backprojector on the fused kernel's traversal (osem.cu). tof == NULL
 // selects the non-TOF rules. Views with equal strides for the two layouts (v x-fastest, vt the
 // optional y-fastest copy).

@@ -230,13 +230,6 @@ k_trace_fused(const float *__restrict__ lors, int64_t n, int stride, const float
                                          SRF_RATIO_PLAIN, 0.0f, v, vt, v, vt, base, false, ll, out);
 }
 
-// The x-dominant in-plane coordinate is divided by dy = (sy / ny) / (sx / nx) in the reference;
-// dy == 1 (square transaxial voxels) makes that division an identity the kernels compile out.
-inline bool grid_qdiv(const Grid &g) {
-    const float dx_ = g.sx / (float)g.nx;
-    return (g.sy / (float)g.ny) / dx_ != 1.0f;
-}
-
 template <int G, bool TOF, int MODE>
 static int launch_trace_fused_g(const float *lors, int64_t n, int stride, const float *tof, int tof_stride,
                                 const Grid &g, const TofParams &tp, const float *values, float *out,

@@ -124,6 +124,22 @@ def backproject(lors: torch.Tensor, values: torch.Tensor, shape, center, size, *
 MAX_BATCH = 8
 
 
+def _width(B: int, shape) -> int:
+    """Values per voxel of the interleaved layout for B images; 0: the separate-image kernels (one image,
+    or so many voxels that element offsets would leave 31 bits)."""
+    w = 0 if B < 2 else 2 if B == 2 else 4 if B <= 4 else 8
+    return w if w * shape[0] * shape[1] * shape[2] < 1 << 31 else 0
+
+
+def _interleaved(shape, width: int, device, fill: bool):
+    """Interleaved buffers: x-fastest, and y-fastest for the y-dominant LORs where a voxel is less than a
+    32-byte sector."""
+    nx, ny, nz = shape
+    new = torch.zeros if fill else torch.empty
+    il = new((nz, ny, nx, width), dtype=F32, device=device)
+    return il, (new((nz, nx, ny, width), dtype=F32, device=device) if width < 8 else None)
+
+
 def project_batch(lors: torch.Tensor, images: torch.Tensor, center, size, *,
                   tof: Optional[Tuple[float, float]] = None, tof_nsigma: float = 0.0) -> torch.Tensor:
     """(B, N) projections of a batch of (nx, ny, nz) images (B <= 8), one traversal per LOR."""
@@ -132,15 +148,27 @@ def project_batch(lors: torch.Tensor, images: torch.Tensor, center, size, *,
     if images.dim() != 4 or not 1 <= images.shape[0] <= MAX_BATCH:
         raise ValueError(f"images must be (B <= {MAX_BATCH}, nx, ny, nz)")
     B, nx, ny, nz = images.shape
-    xb = images.permute(0, 3, 2, 1).contiguous()             # (B, nz, ny, nx): x fastest
-    yb = images.permute(0, 3, 1, 2).contiguous()             # (B, nz, nx, ny): y fastest
     out = torch.empty((B, n), dtype=F32, device=lors.device)
+    if B == 1:
+        project(lors, images[0], center, size, tof=tof, tof_nsigma=tof_nsigma, out=out[0])
+        return out
+    s = stream_ptr(lors.device)
     tof_p = _tof_ptr(lors) if tof is not None else None
     tb, tsg = tof if tof is not None else (0.0, 0.0)
+    w = _width(B, (nx, ny, nz))
+    if w:
+        il, il_t = _interleaved((nx, ny, nz), w, lors.device, fill=False)
+        call("srf_interleave", ptr(images), i64(images.stride(0)), i64x3(images.stride()[1:]), i32(B), i32(w),
+             i32x3((nx, ny, nz)), ptr(il), ptr(il_t), s)
+        call("srf_projection_il", ptr(lors), i64(n), i32(stride), tof_p, i32(stride), *_tof_args(tb, tsg, tof_nsigma),
+             i32(B), i32(w), ptr(il), ptr(il_t), i32x3((nx, ny, nz)), f32x3(center), f32x3(size), ptr(out), i64(n), s)
+        return out
+    xb = images.permute(0, 3, 2, 1).contiguous()             # (B, nz, ny, nx): x fastest
+    yb = images.permute(0, 3, 1, 2).contiguous()             # (B, nz, nx, ny): y fastest
     call("srf_projection_batch", ptr(lors), i64(n), i32(stride), tof_p, i32(stride),
          *_tof_args(tb, tsg, tof_nsigma), i32(B), i64(nx * ny * nz), ptr(xb), i64x3((1, nx, nx * ny)),
          ptr(yb), i64x3((ny, 1, nx * ny)), i32x3((nx, ny, nz)), f32x3(center), f32x3(size), ptr(out),
-         i64(n), stream_ptr(lors.device))
+         i64(n), s)
     return out
 
 
@@ -154,14 +182,27 @@ def adjoint_batch(lors: torch.Tensor, values: torch.Tensor, shape, center, size,
         raise ValueError(f"values must be (B <= {MAX_BATCH}, N)")
     B = values.shape[0]
     nx, ny, nz = shape
-    acc = torch.zeros((B, nz, ny, nx), dtype=F32, device=lors.device)
-    acc_t = torch.zeros((B, nz, nx, ny), dtype=F32, device=lors.device)
+    if B == 1:
+        return backproject(lors, values[0], shape, center, size, tof=tof, tof_nsigma=tof_nsigma, adjoint=True)[None]
+    s = stream_ptr(lors.device)
     tof_p = _tof_ptr(lors) if tof is not None else None
     tb, tsg = tof if tof is not None else (0.0, 0.0)
+    w = _width(B, shape)
+    if w:
+        il, il_t = _interleaved(shape, w, lors.device, fill=True)
+        call("srf_projection_adjoint_il", ptr(lors), i64(n), i32(stride), tof_p, i32(stride),
+             *_tof_args(tb, tsg, tof_nsigma), i32(B), i32(w), ptr(values), i64(n), ptr(il), ptr(il_t), i32x3(shape),
+             f32x3(center), f32x3(size), s)
+        out = torch.empty((B, nx, ny, nz), dtype=F32, device=lors.device)
+        call("srf_deinterleave", ptr(il), ptr(il_t), i32(B), i32(w), i32x3(shape), ptr(out), i64(out.stride(0)),
+             i64x3(out.stride()[1:]), s)
+        return out
+    acc = torch.zeros((B, nz, ny, nx), dtype=F32, device=lors.device)
+    acc_t = torch.zeros((B, nz, nx, ny), dtype=F32, device=lors.device)
     call("srf_projection_adjoint_batch", ptr(lors), i64(n), i32(stride), tof_p, i32(stride),
          *_tof_args(tb, tsg, tof_nsigma), i32(B), ptr(values), i64(n), ptr(acc), i64(nx * ny * nz),
          i64x3((1, nx, nx * ny)), ptr(acc_t), i64x3((ny, 1, nx * ny)), i32x3(shape), f32x3(center),
-         f32x3(size), stream_ptr(lors.device))
+         f32x3(size), s)
     out = acc.permute(0, 3, 2, 1)                             # (B, nx, ny, nz) views, x fastest
     for b in range(B):
         fold(out[b], acc_t[b].permute(1, 2, 0))
