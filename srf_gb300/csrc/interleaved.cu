@@ -113,7 +113,7 @@ k_trace_il(const float *__restrict__ lors, int64_t n, int stride, const float *_
 #pragma unroll
                 for (int c = 0; c < 6; ++c) lv[c] = __ldg(l + c);
                 const float tv = TOF ? __ldg(tof + il * tof_stride) : 0.0f;
-                E = make_lean<TOF>(setup_rec<TOF>(lv, tv, 1.0f, g, k), g, k, v.st, vt.st, have_t);
+                E = make_lean<TOF, 32>(setup_rec<TOF>(lv, tv, 1.0f, g, k), g, k, v.st, vt.st, have_t, 0);
             }
             store_lean(&rec[lane], E);
 #pragma unroll
@@ -148,24 +148,16 @@ k_trace_il(const float *__restrict__ lors, int64_t n, int stride, const float *_
                         });
                 }
             } else if ((!ADJ || any) && (E.flags & F_VALID) && (E.flags & F_PROJ)) {
-                const LeanAxes ax = lean_axes(E, g, v.st, vt.st, have_t);
                 float *im = (!(E.flags & F_XDOM) && have_t) ? vt.ptr : v.ptr;
                 if (ADJ) a = times<W>(a, E.invL2);
-                const int plo = max(E.lo, E.pmlo), phi = min(E.hi, E.pmhi);
-                const float ppmax = (float)(phi - E.ic);
-                int32_t o[U][3];
-                float w[U][3];
-                for (int c0 = plo; c0 <= phi; c0 += 32 * U) {
-                    lean_chunk<TOF, U, 32, QDIV>(E, ax, c0, phi, ppmax, lane, o, w);
-                    if (ADJ) {
+                lean_walk<TOF, U, 32, QDIV>(E, lean_axes(E, g), E.plo, E.phi, lane, [&](auto &o, auto &w, auto ng) {
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
+                    for (int u = 0; u < decltype(ng)::value; ++u) {
+                        if (ADJ) {
 #pragma unroll
                             for (int c = 0; c < 3; ++c)
                                 if (w[u][c] != 0.0f) red_vals<W>(im + o[u][c], times<W>(a, w[u][c]));
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
+                        } else {
                             Vals<W> x[3] = {};
 #pragma unroll
                             for (int c = 0; c < 3; ++c)
@@ -177,7 +169,7 @@ k_trace_il(const float *__restrict__ lors, int64_t n, int stride, const float *_
                                     a.v[b] = __ffma2_rn(x[c].v[b], make_float2(w[u][c], w[u][c]), a.v[b]);
                         }
                     }
-                }
+                });
                 if (!ADJ) a = times<W>(a, E.invL2);
             }
             if (!ADJ) {

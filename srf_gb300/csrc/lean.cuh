@@ -32,12 +32,16 @@
 // the projector's endpoint slab range and the truncated TOF window (t2 <= nsigma^2).
 //
 // Range tests. Per LOR, [ilo, ihi] is the slab range whose face coordinates all lie at least
-// kInteriorMargin inside the image box, so every candidate voxel is inside. A group of 32 slabs
-// entirely within it skips the reference's range tests (siddon.cu.cc:88-189); other groups run
-// them. A chunk whose active groups all lie within it runs them without a branch between them, so
-// that the groups' independent instruction chains interleave. Gathers and reductions are
-// predicated on a non-zero weight (a zero-weight slot still has a valid address, so neither needs
-// a range test).
+// kInteriorMargin inside the image box, so every candidate voxel is inside. Groups of slabs entirely
+// within it skip the reference's range tests (siddon.cu.cc:88-189) and run up to four at a time
+// without a branch between them, so that their instruction chains interleave; other groups run the
+// tests one group at a time. A LOR whose coordinates step more than one voxel per slab (non-square
+// voxels, steep LORs) has no interior. Gathers and reductions are predicated on a non-zero weight (a
+// zero-weight slot of an interior group still has a valid address).
+//
+// Interior groups work on two slabs per lane at a time in packed FP32 (one instruction, two
+// independent roundings, each that of the scalar operation): the loop is bound by instruction issue.
+// Their voxels follow from the first one by per-LOR strides, because a floor moves by at most one.
 #pragma once
 #include "fused.cuh"
 
@@ -50,13 +54,15 @@ constexpr float kInteriorMargin = 0.01f;     // voxel units
 struct __align__(16) LeanRec {
     float invq, invz, Bz, Z1;     // 1/|q step|, 1/|z step| per slab; z faces: fma(Bz, pp, Z1 or Z2)
     float Z2, tS, tT, wc;         // TOF: exponent -(fma(tS, pp, tT))^2 in log2 units; wc with amplitude
-    float invL2, yv, ad, ppmax;   // ppmax = hi - ic
+    float invL2, yv, ad, nq2;
     float p1, q1, kq, dq;         // the q face coordinate in the reference's operand order
-    float rdq, icnp, nq2, pad0;   // rdq = RN(1 / dq); icnp = ic - np/2 (exact)
-    int lo, hi, ic, flags;        // flags: F_VALID | F_PROJ | F_XDOM | F_TIE
-    int ilo, ihi, pmlo, pmhi;     // interior slabs; projector endpoint rule
-    int base, pad1, pad2, pad3;   // element offset of slab ic at the floor-bit origin (mod 2^32)
+    float rdq, c1, c2, neg_zero;  // rdq = RN(1 / dq); pp + c1, pp + c2: faces of the lower and upper q (exact)
+    int lo, hi, ic, flags;        // flags: F_VALID | F_PROJ | F_XDOM | F_TIE | F_HOT, its groups << kHotShift
+    int ilo, ihi, plo, phi;       // interior slabs; the projector's slabs (empty when it skips the LOR)
+    int base, sp, sq, sz;         // element offset of slab ic at the floor-bit origin (mod 2^32); strides
 };
+// F_HOT: the projector's slabs are all of the LOR's, interior, and fit one chunk of the kernel.
+constexpr int F_HOT = 16, kHotShift = 8;
 constexpr int kLeanVec = sizeof(LeanRec) / 16;
 static_assert(sizeof(LeanRec) == 128, "LeanRec is eight 16-byte vectors");
 
@@ -80,27 +86,28 @@ __device__ __forceinline__ void store_lean(LeanRec *dst, const LeanRec &R) {
 // (siddon_tof.cu.cc:55-58: xc, d2_tof, t2), as the oracle applies it.
 __device__ __forceinline__ bool tof_keep(const LorRec &R, const GridK &k, int ip, int np_half, float dpc) {
     const float pc = __fmul_rn(__fadd_rn((float)(ip - np_half), 0.5f), dpc);
-    const float d2 = __fmul_rn(__fsub_rn(__fdiv_rn(__fsub_rn(pc, R.p1), R.pd), R.ratio1), R.L);
-    const float t2 = __fdiv_rn(__fmul_rn(d2, d2), k.expand);
+    const float d2 = __fmul_rn(__fsub_rn(div_exact(__fsub_rn(pc, R.p1), R.pd, R.rpd), R.ratio1), R.L);
+    const float t2 = div_exact(__fmul_rn(d2, d2), k.expand, k.rexp);
     return t2 <= k.nsig2;
 }
 
 // [a, b] of real face positions f where A + B f stays within [m, n - m] (its FP32 rounding is far
-// inside the margin m).
-__device__ __forceinline__ void face_interval(float A, float B, float n, float m, float &a, float &b) {
+// inside the margin m); rB = 1 / B.
+__device__ __forceinline__ void face_interval(float A, float B, float rB, float n, float m, float &a, float &b) {
     if (B == 0.0f) {
         if (A >= m && A <= n - m) { a = -1e30f; b = 1e30f; } else { a = 1e30f; b = -1e30f; }
         return;
     }
-    const float t1 = (m - A) / B, t2 = (n - m - A) / B;
+    const float t1 = (m - A) * rB, t2 = (n - m - A) * rB;
     a = fminf(t1, t2);
     b = fmaxf(t1, t2);
 }
 
-// Lean record of a LOR from its setup record (lane-parallel, once per LOR).
-template <bool TOF>
+// Lean record of a LOR from its setup record (lane-parallel, once per LOR). hot: slabs of one chunk of
+// the kernel that walks it (0: no F_HOT), G: its lanes per LOR.
+template <bool TOF, int G>
 __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, const GridK &k,
-                                             const int64_t stx[3], const int64_t sty[3], bool have_t) {
+                                             const int64_t stx[3], const int64_t sty[3], bool have_t, int hot) {
     LeanRec E = {};
     E.flags = R.flags;
     E.yv = R.yv;
@@ -108,8 +115,7 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
     E.invL2 = R.invL2;
     E.lo = R.lo;
     E.hi = R.hi;
-    E.pmlo = R.pmlo;
-    E.pmhi = R.pmhi;
+    E.plo = 1;
     if (!(R.flags & F_VALID) || (R.flags & F_TIE)) return E;
     const bool xdom = R.flags & F_XDOM;
     const int np = xdom ? g.nx : g.ny, nq = xdom ? g.ny : g.nx;
@@ -117,14 +123,15 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
     const int np_half = np / 2;
     const float dpc = xdom ? 1.0f : k.dy;
     // d(ip) = ((pc(ip) - p1) / pd - ratio1) L with pc(ip) = (ip - np/2 + 0.5) dpc is linear in ip
-    const float tA = dpc / R.pd * R.L;
+    const float tA = div_exact(dpc, R.pd, R.rpd) * R.L;
     int lo = R.lo, hi = R.hi;
     if (TOF && k.nsig2 > 0.0f && lo <= hi) {
         // exact truncated window: t2 <= nsigma^2 keeps an interval of slabs; estimate it (to a
         // slab) and settle both ends with the predicate itself
-        const float tB = (((0.5f - (float)np_half) * dpc - R.p1) / R.pd - R.ratio1) * R.L;
-        const float half = sqrtf(k.nsig2 * k.expand) / fabsf(tA);
-        const float c = -tB / tA;
+        const float tB = (((0.5f - (float)np_half) * dpc - R.p1) * R.rpd - R.ratio1) * R.L;
+        const float rtA = __fdividef(1.0f, tA);
+        const float half = k.nsw * fabsf(rtA);
+        const float c = -tB * rtA;
         int a = (int)fmaxf(fminf(ceilf(c - half), (float)hi + 1.0f), (float)lo - 1.0f);
         int b = (int)fmaxf(fminf(floorf(c + half), (float)hi + 1.0f), (float)lo - 1.0f);
         for (int t = 0; t < 6 && a > lo && tof_keep(R, k, a - 1, np_half, dpc); ++t) --a;
@@ -142,7 +149,6 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
     E.hi = hi;
     const int ic = (lo + hi) >> 1;
     E.ic = ic;
-    E.ppmax = (float)(hi - ic);
     // z at face f (slab ip has faces ip and ip + 1): Az + Bz (f - np/2); at pp = ip - ic the
     // lower face is f = ip + (Bz < 0), the upper one f = ip + (Bz >= 0)
     const float icnp = __fsub_rn((float)ic, np2);  // exact
@@ -150,95 +156,107 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
     E.Bz = R.Bz;
     E.Z1 = fmaf(R.Bz, icnp + s_lo, R.Az);
     E.Z2 = fmaf(R.Bz, icnp + (1.0f - s_lo), R.Az);
-    E.invq = R.invq;
-    E.invz = R.invz;
+    E.invq = fabsf(R.rBq);
+    E.invz = fabsf(R.rBz);
     E.wc = R.wc;
     E.p1 = R.p1;
     E.q1 = R.q1;
     E.kq = R.kq;
     E.dq = xdom ? k.dy : 1.0f;
-    E.rdq = __frcp_rn(E.dq);
-    E.icnp = icnp;
+    E.rdq = xdom ? k.rdy : 1.0f;
+    E.c1 = icnp + (R.kq >= 0.0f ? 0.0f : 1.0f);
+    E.c2 = icnp + (R.kq >= 0.0f ? 1.0f : 0.0f);
     E.nq2 = xdom ? k.ny2 : k.nx2;
+    E.neg_zero = -0.0f;
     if (TOF) {
         // exponent of the Gaussian in log2 units: d(ip)^2 k2 = -(s d(ip))^2, s = sqrt(-k2), with
         // d = tA pp + d(ic), d(ic) in the reference's operand order
         const float s = sqrtf(-k.k2);
         const float pc = __fmul_rn(__fadd_rn((float)(ic - np_half), 0.5f), dpc);
-        const float dic = __fmul_rn(__fsub_rn(__fdiv_rn(__fsub_rn(pc, R.p1), R.pd), R.ratio1), R.L);
+        const float dic = __fmul_rn(__fsub_rn(div_exact(__fsub_rn(pc, R.p1), R.pd, R.rpd), R.ratio1), R.L);
         E.tS = tA * s;
         E.tT = dic * s;
     }
     // interior slabs: both faces of every slab within the box by the margin, in q and in z
     float qa, qb, za, zb;
-    face_interval(R.Aq - R.Bq * np2, R.Bq, (float)nq, kInteriorMargin, qa, qb);
-    face_interval(R.Az - R.Bz * np2, R.Bz, (float)g.nz, kInteriorMargin, za, zb);
+    face_interval(R.Aq - R.Bq * np2, R.Bq, R.rBq, (float)nq, kInteriorMargin, qa, qb);
+    face_interval(R.Az - R.Bz * np2, R.Bz, R.rBz, (float)g.nz, kInteriorMargin, za, zb);
     const float fa = fmaxf(qa, za), fb = fminf(qb, zb);   // faces f in [fa, fb]
     const float il = fmaxf(ceilf(fa), (float)lo), ih = fminf(floorf(fb) - 1.0f, (float)hi);
-    E.ilo = il <= ih ? (int)il : 1;
-    E.ihi = il <= ih ? (int)ih : 0;
+    const bool inner = il <= ih && fabsf(R.Bq) <= 1.0f + 1e-5f && fabsf(R.Bz) <= 1.0f + 1e-5f;
+    E.ilo = inner ? (int)il : 1;
+    E.ihi = inner ? (int)ih : 0;
+    E.plo = (R.flags & F_PROJ) ? max(lo, R.pmlo) : 1;
+    E.phi = (R.flags & F_PROJ) ? min(hi, R.pmhi) : 0;
+    if (E.plo == lo && E.phi == hi && lo >= E.ilo && hi <= E.ihi && hi - lo < hot)
+        E.flags |= F_HOT | (((hi - lo) / G + 1) << kHotShift);
     // element offset of (slab ic, floor bits 0x4B400000 + cq, 0x4B400000 + cz), modulo 2^32
     const int64_t *st = (!xdom && have_t) ? sty : stx;
     const uint32_t sp = (uint32_t)(xdom ? st[0] : st[1]);
     const uint32_t sq = (uint32_t)(xdom ? st[1] : st[0]);
     const uint32_t sz = (uint32_t)st[2];
     E.base = (int)((uint32_t)ic * sp - (uint32_t)kFloorBits * (sq + sz));
+    E.sp = (int)sp;
+    E.sq = (int)sq;
+    E.sz = (int)sz;
     return E;
 }
 
-// Per-lane strides of the LOR's view and grid extents (no per-slab selects).
+// Extents of the LOR's in-plane secondary and axial directions (the range tests').
 struct LeanAxes {
-    int32_t sp, sq, sz, nq, nz;
+    int32_t nq, nz;
 };
 
-__device__ __forceinline__ LeanAxes lean_axes(const LeanRec &E, const Grid &g, const int64_t stx[3],
-                                              const int64_t sty[3], bool have_t) {
-    const bool xdom = E.flags & F_XDOM;
-    const int64_t *st = (!xdom && have_t) ? sty : stx;
-    LeanAxes a;
-    a.sp = (int32_t)(xdom ? st[0] : st[1]);
-    a.sq = (int32_t)(xdom ? st[1] : st[0]);
-    a.sz = (int32_t)st[2];
-    a.nq = xdom ? g.ny : g.nx;
-    a.nz = g.nz;
-    return a;
+__device__ __forceinline__ LeanAxes lean_axes(const LeanRec &E, const Grid &g) {
+    return LeanAxes{(E.flags & F_XDOM) ? g.ny : g.nx, g.nz};
 }
 
-// a / b correctly rounded from rb = RN(1 / b): one Newton step on the residual, which the FMA
-// computes exactly (Markstein's division; a / 1 returns a unchanged)
-__device__ __forceinline__ float div_refined(float a, float b, float rb) {
-    const float q0 = __fmul_rn(a, rb);
-    const float r = __fmaf_rn(-q0, b, a);
-    return __fmaf_rn(r, rb, q0);
+// float and float2 (two slabs, packed instructions) forms of the slab arithmetic
+__device__ __forceinline__ float f_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float f_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float f_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float f_add_rd(float a, float b) { return __fadd_rd(a, b); }
+__device__ __forceinline__ float2 f_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 f_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 f_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 f_add_rd(float2 a, float2 b) { return __fadd2_rd(a, b); }
+template <typename T> __device__ __forceinline__ T f_all(float a);
+template <> __device__ __forceinline__ float f_all<float>(float a) { return a; }
+template <> __device__ __forceinline__ float2 f_all<float2>(float a) { return make_float2(a, a); }
+template <typename T> constexpr int kParts = sizeof(T) / sizeof(float);
+__device__ __forceinline__ float part(float a, int) { return a; }
+__device__ __forceinline__ float part(float2 a, int i) { return i ? a.y : a.x; }
+__device__ __forceinline__ void set_part(float &a, int, float v) { a = v; }
+__device__ __forceinline__ void set_part(float2 &a, int i, float v) { if (i) a.y = v; else a.x = v; }
+// A product that a following sum must not absorb: the compiler fuses a packed product and sum even where
+// both are rounded explicitly (seen as q faces off by one rounding), so the packed product is an FMA with
+// a -0 that the compiler cannot see.
+__device__ __forceinline__ float f_mul_rounded(float a, float b, float) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float2 f_mul_rounded(float2 a, float2 b, float neg_zero) {
+    return __ffma2_rn(a, b, make_float2(neg_zero, neg_zero));
 }
 
-// The slab's q face coordinates (qq1 <= qq2) in the reference's operand order
-// (siddon.cu.cc:59-73: (q1 + kq (pp - p1)) / dq + nq2 at pp = ip - np/2 and ip - np/2 + 1), so
-// that the q floors and crossing fractions are the reference's. QDIV: dq != 1 (non-square
-// transaxial voxels, x-dominant LORs).
-template <bool QDIV>
-__device__ __forceinline__ void q_faces(const LeanRec &E, float pp, float &qq1, float &qq2) {
-    const float ppf = __fadd_rn(pp, E.icnp);  // ip - np/2, exact
-    float ta = __fadd_rn(E.q1, __fmul_rn(E.kq, __fsub_rn(ppf, E.p1)));
-    float tb = __fadd_rn(E.q1, __fmul_rn(E.kq, __fsub_rn(__fadd_rn(ppf, 1.0f), E.p1)));
+// The slab's q face coordinate at pp + c in the reference's operand order (siddon.cu.cc:59-73:
+// (q1 + kq (pp - p1)) / dq + nq2 at pp = ip - np/2 or ip - np/2 + 1), so that the q floors and crossing
+// fractions are the reference's. QDIV: dq != 1 (non-square transaxial voxels, x-dominant LORs); the
+// division is one Newton step from rdq = RN(1 / dq) (Markstein; a / 1 returns a unchanged).
+template <bool QDIV, typename T>
+__device__ __forceinline__ T q_face(const LeanRec &E, T pp, float c) {
+    T t = f_add(f_all<T>(E.q1), f_mul_rounded(f_all<T>(E.kq), f_add(f_add(pp, f_all<T>(c)), f_all<T>(-E.p1)), E.neg_zero));
     if (QDIV) {
-        ta = div_refined(ta, E.dq, E.rdq);
-        tb = div_refined(tb, E.dq, E.rdq);
+        const T q0 = f_mul(t, f_all<T>(E.rdq));
+        const T r = f_fma(q0, f_all<T>(-E.dq), t);
+        t = f_fma(r, f_all<T>(E.rdq), q0);
     }
-    ta = __fadd_rn(ta, E.nq2);
-    tb = __fadd_rn(tb, E.nq2);
-    const bool up = E.kq >= 0.0f;
-    qq1 = up ? ta : tb;
-    qq2 = up ? tb : ta;
+    return f_add(t, f_all<T>(E.nq2));
 }
 
-// One slab of a LOR: the three slots' element offsets and weights (zero for a voxel the slab
-// does not visit). ipc = min(ip, hi); act = ip <= hi (an inactive lane contributes zero weight
-// at a valid address). EDGE runs the reference's range tests; without it the caller guarantees
-// that ipc lies in [ilo, ihi].
-template <bool TOF, bool EDGE, bool QDIV>
-__device__ __forceinline__ void lean_slab(const LeanRec &E, const LeanAxes &ax, int ipc, float pp, bool act,
-                                          int32_t o[3], float w[3]) {
+// One slab near the image faces: the three slots' element offsets and weights (zero for a voxel the
+// slab does not visit) under the reference's range tests. ipc = min(ip, hi); act = ip <= hi (an
+// inactive lane contributes zero weight).
+template <bool TOF, bool QDIV>
+__device__ __forceinline__ void lean_slab(const LeanRec &E, const LeanAxes &ax, int ipc, bool act, int32_t o[3], float w[3]) {
+    const float pp = (float)(ipc - E.ic);
     float wt = E.wc;
     if (TOF) {
         const float d = fmaf(E.tS, pp, E.tT);
@@ -247,8 +265,7 @@ __device__ __forceinline__ void lean_slab(const LeanRec &E, const LeanAxes &ax, 
         wt *= ex;
     }
     wt = act ? wt : 0.0f;
-    float qq1, qq2;
-    q_faces<QDIV>(E, pp, qq1, qq2);
+    const float qq1 = q_face<QDIV>(E, pp, E.c1), qq2 = q_face<QDIV>(E, pp, E.c2);
     const float zz1 = fmaf(E.Bz, pp, E.Z1), zz2 = fmaf(E.Bz, pp, E.Z2);
     const float fq1 = __fadd_rd(qq1, kFloorMagic), fq2 = __fadd_rd(qq2, kFloorMagic);
     const float fz1 = __fadd_rd(zz1, kFloorMagic), fz2 = __fadd_rd(zz2, kFloorMagic);
@@ -259,90 +276,177 @@ __device__ __forceinline__ void lean_slab(const LeanRec &E, const LeanAxes &ax, 
     const float fz = dz ? ((fz2 - kFloorMagic) - zz1) * E.invz : 1.0f;
     const bool qfirst = fq > fz;
     const float mn = fminf(fq, fz), mx = fmaxf(fq, fz);
-    float w0 = mn * wt, w1 = fabsf(fq - fz) * wt, w2 = fmaf(-mx, wt, wt);
-    const uint32_t base = (uint32_t)E.base + (uint32_t)(ipc - E.ic) * (uint32_t)ax.sp;
-    const uint32_t t1 = (uint32_t)bz1 * (uint32_t)ax.sz + base;
-    const uint32_t t2 = (uint32_t)bz2 * (uint32_t)ax.sz + base;
-    int32_t o0 = (int32_t)((uint32_t)bq1 * (uint32_t)ax.sq + t1);
-    const int32_t oa = (int32_t)((uint32_t)bq2 * (uint32_t)ax.sq + t1);   // (cq2, cz1)
-    const int32_t ob = (int32_t)((uint32_t)bq1 * (uint32_t)ax.sq + t2);   // (cq1, cz2)
-    int32_t o2 = (int32_t)((uint32_t)bq2 * (uint32_t)ax.sq + t2);
-    int32_t o1 = qfirst ? ob : oa;
-    if (EDGE) {
-        // the reference's range tests (cq1 <= cq2, cz1 <= cz2): c in [0, n) as one unsigned compare
-        const bool A = (unsigned)(bq1 - kFloorBits) < (unsigned)ax.nq;
-        const bool B = (unsigned)(bz1 - kFloorBits) < (unsigned)ax.nz;
-        const bool C = (unsigned)(bq2 - kFloorBits) < (unsigned)ax.nq;
-        const bool D = (unsigned)(bz2 - kFloorBits) < (unsigned)ax.nz;
-        const bool qm = bq1 >= kFloorBits - 1, zm = bz1 >= kFloorBits - 1;
-        const bool v0 = A && B;
-        const bool v1 = qfirst ? (A && D && zm) : (C && B && qm);
-        const bool v2 = C && D && qm && zm;
-        w0 = v0 ? w0 : 0.0f;
-        w1 = v1 ? w1 : 0.0f;
-        w2 = v2 ? w2 : 0.0f;
-        o0 = v0 ? o0 : 0;
-        o1 = v1 ? o1 : 0;
-        o2 = v2 ? o2 : 0;
-    }
-    o[0] = o0; o[1] = o1; o[2] = o2;
-    w[0] = w0; w[1] = w1; w[2] = w2;
+    const float w0 = mn * wt, w1 = fabsf(fq - fz) * wt, w2 = fmaf(-mx, wt, wt);
+    const uint32_t base = (uint32_t)E.base + (uint32_t)(ipc - E.ic) * (uint32_t)E.sp;
+    const uint32_t t1 = (uint32_t)bz1 * (uint32_t)E.sz + base;
+    const uint32_t t2 = (uint32_t)bz2 * (uint32_t)E.sz + base;
+    const uint32_t oa = (uint32_t)bq2 * (uint32_t)E.sq + t1;   // (cq2, cz1)
+    const uint32_t ob = (uint32_t)bq1 * (uint32_t)E.sq + t2;   // (cq1, cz2)
+    // the reference's range tests (cq1 <= cq2, cz1 <= cz2): c in [0, n) as one unsigned compare
+    const bool A = (unsigned)(bq1 - kFloorBits) < (unsigned)ax.nq;
+    const bool B = (unsigned)(bz1 - kFloorBits) < (unsigned)ax.nz;
+    const bool C = (unsigned)(bq2 - kFloorBits) < (unsigned)ax.nq;
+    const bool D = (unsigned)(bz2 - kFloorBits) < (unsigned)ax.nz;
+    const bool qm = bq1 >= kFloorBits - 1, zm = bz1 >= kFloorBits - 1;
+    w[0] = A && B ? w0 : 0.0f;
+    w[1] = (qfirst ? (A && D && zm) : (C && B && qm)) ? w1 : 0.0f;
+    w[2] = C && D && qm && zm ? w2 : 0.0f;
+    o[0] = (int32_t)((uint32_t)bq1 * (uint32_t)E.sq + t1);
+    o[1] = (int32_t)(qfirst ? ob : oa);
+    o[2] = (int32_t)((uint32_t)bq2 * (uint32_t)E.sq + t2);
 }
 
-// The first N groups of a chunk, all inside [ilo, ihi], as straight-line code (no branch
-// between the groups, so their instruction streams interleave); groups N..U-1 are zero.
-template <bool TOF, int U, int G, bool QDIV, int N>
-__device__ __forceinline__ void lean_interior_groups(const LeanRec &E, const LeanAxes &ax, int c0, int whi,
-                                                     float ppmax, float pp0, int lane, int32_t (&o)[U][3],
-                                                     float (&w)[U][3]) {
+// kParts<T> interior slabs of this lane (both faces inside the box, floors that move by at most one):
+// pp and the element offset at the floor-bit origin of each; act_last: whether the last is the LOR's.
+template <bool TOF, bool QDIV, typename T>
+__device__ __forceinline__ void interior_slabs(const LeanRec &E, T pp, const uint32_t *base, bool act_last,
+                                               int32_t (*o)[3], float (*w)[3]) {
+    constexpr int P = kParts<T>;
+    T wt = f_all<T>(E.wc);
+    if (TOF) {
+        const T d = f_fma(f_all<T>(E.tS), pp, f_all<T>(E.tT));
+        const T dd = f_mul(d, d);
+        T ex;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        if (u < N) {
-            const int ip = c0 + G * u + lane;
-            const bool act = ip <= whi;
-            lean_slab<TOF, false, QDIV>(E, ax, act ? ip : whi, fminf(pp0 + (float)(G * u), ppmax), act, o[u], w[u]);
+        for (int i = 0; i < P; ++i) {
+            float v;
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v) : "f"(-part(dd, i)));
+            set_part(ex, i, v);
+        }
+        wt = f_mul(wt, ex);
+    }
+    set_part(wt, P - 1, act_last ? part(wt, P - 1) : 0.0f);
+    const T qq1 = q_face<QDIV>(E, pp, E.c1), qq2 = q_face<QDIV>(E, pp, E.c2);
+    const T zz1 = f_fma(f_all<T>(E.Bz), pp, f_all<T>(E.Z1)), zz2 = f_fma(f_all<T>(E.Bz), pp, f_all<T>(E.Z2));
+    const T M = f_all<T>(kFloorMagic), Mn = f_all<T>(-kFloorMagic), one_m = f_all<T>(-1.0f);
+    const T fq1 = f_add_rd(qq1, M), fq2 = f_add_rd(qq2, M), fz1 = f_add_rd(zz1, M), fz2 = f_add_rd(zz2, M);
+    const T rq = f_mul(f_fma(qq1, one_m, f_add(fq2, Mn)), f_all<T>(E.invq));
+    const T rz = f_mul(f_fma(zz1, one_m, f_add(fz2, Mn)), f_all<T>(E.invz));
+    T fq, fz, mn, mx;
+    uint32_t step_q[P], step_z[P];  // from the first voxel across the crossings there are
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+        const bool dq = part(fq1, i) != part(fq2, i), dz = part(fz1, i) != part(fz2, i);
+        const float a = dq ? part(rq, i) : 1.0f, b = dz ? part(rz, i) : 1.0f;
+        step_q[i] = dq ? (uint32_t)E.sq : 0u;
+        step_z[i] = dz ? (uint32_t)E.sz : 0u;
+        set_part(fq, i, a);
+        set_part(fz, i, b);
+        set_part(mn, i, fminf(a, b));
+        set_part(mx, i, fmaxf(a, b));
+    }
+    const T w0 = f_mul(mn, wt), w2 = f_fma(mx, f_mul(wt, one_m), wt);
+    const T w1 = f_mul(f_fma(fz, one_m, fq), wt);  // > 0: slot 1 is (cq1, cz2), else (cq2, cz1)
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+        const uint32_t o0 = (uint32_t)__float_as_int(part(fq1, i)) * (uint32_t)E.sq +
+                            ((uint32_t)__float_as_int(part(fz1, i)) * (uint32_t)E.sz + base[i]);
+        o[i][0] = (int32_t)o0;
+        // a fraction can round to just above 1 (a crossing at the slab's far face): slot 1 or 2 then has a
+        // weight of the order of that rounding, at a voxel that the slab touches
+        o[i][1] = (int32_t)(o0 + (part(w1, i) > 0.0f ? step_z[i] : step_q[i]));
+        o[i][2] = (int32_t)(o0 + step_z[i] + step_q[i]);
+        w[i][0] = part(w0, i);
+        w[i][1] = fabsf(part(w1, i));
+        w[i][2] = part(w2, i);
+    }
+}
+
+// N interior groups of G slabs from slab c0, the last one cut at whi (the others are whole).
+template <bool TOF, int G, bool QDIV, int N>
+__device__ __forceinline__ void interior_groups(const LeanRec &E, int c0, int whi, int lane, int32_t (*o)[3], float (*w)[3]) {
+    const int ip = c0 + lane, last = ip + G * (N - 1);
+    const bool act = last <= whi;
+    const float pp0 = (float)(ip - E.ic);
+    uint32_t base[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+        base[u] = (uint32_t)E.base + (uint32_t)((u == N - 1 ? min(last, whi) : ip + G * u) - E.ic) * (uint32_t)E.sp;
+    const float pp_last = fminf(pp0 + (float)(G * (N - 1)), (float)(whi - E.ic));
+#pragma unroll
+    for (int u = 0; u + 1 < N; u += 2) {
+        const float2 pp = make_float2(pp0 + (float)(G * u), u + 2 == N ? pp_last : pp0 + (float)(G * (u + 1)));
+        interior_slabs<TOF, QDIV, float2>(E, pp, base + u, u + 2 == N ? act : true, o + u, w + u);
+    }
+    if (N & 1) interior_slabs<TOF, QDIV, float>(E, pp_last, base + N - 1, act, o + N - 1, w + N - 1);
+}
+
+template <int N> struct Groups { static constexpr int value = N; };
+
+// A walk over slabs [lo, hi] of a LOR with G lanes: f(o, w, Groups<N>) for every run of N <= U interior
+// groups and every edge group.
+template <bool TOF, int U, int G, bool QDIV, typename F>
+__device__ __forceinline__ void lean_walk(const LeanRec &E, const LeanAxes &ax, int lo, int hi, int lane, F &&f) {
+    static_assert(U >= 1 && U <= 4, "1 to 4 groups per run");
+    int32_t o[U][3];
+    float w[U][3];
+    for (int c = lo; c <= hi;) {
+        // whole interior groups from c (the last one may be cut at hi)
+        const int n = c < E.ilo ? 0 : E.ihi >= hi ? (hi - c) / G + 1 : (E.ihi - c + 1) / G;
+        if (n >= U) {
+            interior_groups<TOF, G, QDIV, U>(E, c, hi, lane, o, w);
+            f(o, w, Groups<U>());
+            c += G * U;
+        } else if (U > 3 && n == 3) {
+            interior_groups<TOF, G, QDIV, (U > 3 ? 3 : 1)>(E, c, hi, lane, o, w);
+            f(o, w, Groups<(U > 3 ? 3 : 1)>());
+            c += G * 3;
+        } else if (U > 2 && n == 2) {
+            interior_groups<TOF, G, QDIV, (U > 2 ? 2 : 1)>(E, c, hi, lane, o, w);
+            f(o, w, Groups<(U > 2 ? 2 : 1)>());
+            c += G * 2;
+        } else if (U > 1 && n == 1) {
+            interior_groups<TOF, G, QDIV, 1>(E, c, hi, lane, o, w);
+            f(o, w, Groups<1>());
+            c += G;
         } else {
-            o[u][0] = o[u][1] = o[u][2] = 0;
-            w[u][0] = w[u][1] = w[u][2] = 0.0f;
+            const int ip = c + lane;
+            lean_slab<TOF, QDIV>(E, ax, min(ip, hi), ip <= hi, o[0], w[0]);
+            f(o, w, Groups<1>());
+            c += G;
         }
     }
 }
 
-// U slabs of one chunk of a walk over slabs [c0, whi] with G lanes per LOR (slab
-// c0 + lane + G u): offsets and weights. Groups of G slabs past whi are skipped; groups inside
-// [ilo, ihi] skip the range tests. When every group with an active slab is inside, one switch on
-// their number runs them as straight-line code.
+// The groups of one chunk [c0, whi] (whi - c0 < G U) with their range tests: offsets and weights of all
+// at once, for a caller that needs them twice; groups past whi have zero weights.
 template <bool TOF, int U, int G, bool QDIV>
-__device__ __forceinline__ void lean_chunk(const LeanRec &E, const LeanAxes &ax, int c0, int whi, float ppmax,
-                                           int lane, int32_t (&o)[U][3], float (&w)[U][3]) {
-    const float pp0 = (float)(c0 + lane - E.ic);
-    const int ng = min(U, (whi - c0) / G + 1);  // groups with an active slab (c0 <= whi)
-    if (c0 >= E.ilo && min(c0 + G * ng - 1, whi) <= E.ihi) {
-        static_assert(U >= 1 && U <= 4, "1 to 4 groups per chunk");
-        switch (ng) {
-        case 1: lean_interior_groups<TOF, U, G, QDIV, 1>(E, ax, c0, whi, ppmax, pp0, lane, o, w); return;
-        case 2: lean_interior_groups<TOF, U, G, QDIV, (U >= 2 ? 2 : 1)>(E, ax, c0, whi, ppmax, pp0, lane, o, w); return;
-        case 3: lean_interior_groups<TOF, U, G, QDIV, (U >= 3 ? 3 : 1)>(E, ax, c0, whi, ppmax, pp0, lane, o, w); return;
-        default: lean_interior_groups<TOF, U, G, QDIV, U>(E, ax, c0, whi, ppmax, pp0, lane, o, w); return;
-        }
-    }
+__device__ __forceinline__ void edge_chunk(const LeanRec &E, const LeanAxes &ax, int c0, int whi, int lane,
+                                           int32_t (&o)[U][3], float (&w)[U][3]) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        const int g0 = c0 + G * u;  // first slab of the group (uniform over the group)
-        if (g0 > whi) {
-            o[u][0] = o[u][1] = o[u][2] = 0;
+        const int ip = c0 + G * u + lane;
+        if (c0 + G * u > whi) {  // uniform over the group
             w[u][0] = w[u][1] = w[u][2] = 0.0f;
+            o[u][0] = o[u][1] = o[u][2] = 0;
             continue;
         }
-        const int ip = g0 + lane;
-        const bool act = ip <= whi;
-        const int ipc = act ? ip : whi;
-        const float pp = fminf(pp0 + (float)(G * u), ppmax);
-        if (g0 >= E.ilo && min(g0 + G - 1, whi) <= E.ihi)
-            lean_slab<TOF, false, QDIV>(E, ax, ipc, pp, act, o[u], w[u]);
-        else
-            lean_slab<TOF, true, QDIV>(E, ax, ipc, pp, act, o[u], w[u]);
+        lean_slab<TOF, QDIV>(E, ax, min(ip, whi), ip <= whi, o[u], w[u]);
     }
+}
+
+// Sum of im * w over the slots of N groups; im += r * w over them.
+template <int N>
+__device__ __forceinline__ float gather_slots(const float *__restrict__ im, const int32_t (*o)[3], const float (*w)[3], float acc) {
+    float x[N][3];
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[u][c] = w[u][c] != 0.0f ? __ldg(im + o[u][c]) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc = fmaf(x[u][c], w[u][c], acc);
+    return acc;
+}
+
+template <int N>
+__device__ __forceinline__ void scatter_slots(float *im, const int32_t (*o)[3], const float (*w)[3], float r) {
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            if (w[u][c] != 0.0f) atomicAdd(im + o[u][c], r * w[u][c]);
 }
 
 }  // namespace srf

@@ -28,14 +28,14 @@ __device__ __forceinline__ float tie_project(const float *l, float tv, int lane,
     return group_sum<G>(acc);
 }
 
-template <int G, bool TOF>
+template <int G, bool TOF, int RULES>
 __device__ __forceinline__ void tie_backproject(const float *l, float tv, float r, int lane, const Grid &g,
                                                 const TofParams &tp, const View &bp, const View &bpt) {
     LorSetup S;
-    if (r != 0.0f && setup_lor<TOF, RULES_BACK>(l[0], l[1], l[2], l[3], l[4], l[5], tv, g, tp, bp.st, bpt.st, bpt.ptr != nullptr, S)) {
+    if (r != 0.0f && setup_lor<TOF, RULES>(l[0], l[1], l[2], l[3], l[4], l[5], tv, g, tp, bp.st, bpt.st, bpt.ptr != nullptr, S)) {
         float *im = (!S.xdom && bpt.ptr) ? bpt.ptr : bp.ptr;
         for (int ip = S.lo + lane; ip <= S.hi; ip += G)
-            slab<TOF, RULES_BACK>(S, ip, [&](int32_t off, float w) { atomicAdd(im + off, r * w); });
+            slab<TOF, RULES>(S, ip, [&](int32_t off, float w) { atomicAdd(im + off, r * w); });
     }
 }
 
@@ -48,18 +48,39 @@ __device__ __forceinline__ void tie_path(const float *l, float tv, float yv, flo
     const float den = __fadd_rn(__fadd_rn(p, ad), eps);
     const float r = (rule == SRF_RATIO_DIV_NO_NAN) ? ((den == 0.0f) ? 0.0f : __fdiv_rn(yv, den)) : __fdiv_rn(yv, den);
     if (want_ll && lane == 0 && den > 0.0f) ll += (double)yv * log((double)den);  // FP64 term and sum
-    tie_backproject<G, TOF>(l, tv, r, lane, g, tp, bp, bpt);
+    tie_backproject<G, TOF, RULES_BACK>(l, tv, r, lane, g, tp, bp, bpt);
 }
 
-// What a traversal of osem_warp_batch does per LOR: the fused OSEM step, or one of its two halves
-// on its own (the projector into out[i], or the backprojector of the values passed as y).
+// What a traversal of osem_warp_batch does per LOR: the fused OSEM step, one of its two halves on its
+// own (the projector into out[i], or the backprojector of the values passed as y), or the projector's
+// exact adjoint (its rules and 1/L^2 weights, scattering the values).
 enum TraceMode : int { MODE_FUSED = 0, MODE_PROJ = 1, MODE_BACK = 2, MODE_ADJ = 3 };
 
-// LORs [base, base + 32) of one study: lane-parallel setup of the 32 records into wrecs, then
-// the warp's 32/G groups walk them (projection, ratio, backprojection per LOR) on the lean slab
-// loop (lean.cuh). x/x_t and bp/bp_t have equal strides (offsets are computed once for the
-// gather and the scatter). The projection walks the slabs the projector's endpoint rule keeps;
-// when that is the whole slab range and it fits one chunk of G*U slabs (the usual case with a
+__device__ __forceinline__ float ratio_of(float yv, float den, int rule) {
+    if (rule == SRF_RATIO_DIV_NO_NAN) return (den == 0.0f) ? 0.0f : __fdiv_rn(yv, den);
+    return __fdiv_rn(yv, den);
+}
+
+// The fused step of a LOR whose N groups are all interior (F_HOT): one straight line from the slabs'
+// arithmetic over the gathers and the ratio to the reductions.
+template <int G, bool TOF, bool QDIV, int N>
+__device__ __forceinline__ void hot_lor(const LeanRec &E, int lane, const float *xim, float *bim, int rule, float eps,
+                                        double &ll, bool want_ll) {
+    int32_t o[N][3];
+    float w[N][3];
+    interior_groups<TOF, G, QDIV, N>(E, E.lo, E.hi, lane, o, w);
+    const float p = group_sum<G>(gather_slots<N>(xim, o, w, 0.0f)) * E.invL2;
+    const float den = __fadd_rn(__fadd_rn(p, E.ad), eps);
+    const float r = ratio_of(E.yv, den, rule);
+    if (want_ll && lane == 0 && den > 0.0f) ll += (double)E.yv * log((double)den);  // FP64 term and sum
+    if (r != 0.0f) scatter_slots<N>(bim, o, w, r);
+}
+
+// LORs [base, base + batch) of one study (batch <= 32, a multiple of 32 / G): lane-parallel setup of
+// the records into wrecs, then the warp's 32/G groups walk them (projection, ratio, backprojection per
+// LOR) on the lean slab loop (lean.cuh). x/x_t and bp/bp_t have equal strides (offsets are computed
+// once for the gather and the scatter). The projection walks the slabs the projector's endpoint rule
+// keeps; when that is the whole slab range and it fits one chunk of G*U slabs (the usual case with a
 // truncated TOF kernel), the backprojection reuses the chunk's offsets and weights.
 template <int G, bool TOF, int U, int MODE = MODE_FUSED, bool QDIV = false>
 __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__restrict__ lors,
@@ -69,17 +90,18 @@ __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__r
                                                 const float *__restrict__ add, int rule, float eps,
                                                 const View &x, const View &xt,
                                                 const View &bp, const View &bpt, int64_t base,
-                                                bool want_ll, double &ll, float *__restrict__ out = nullptr) {
+                                                bool want_ll, double &ll, float *__restrict__ out = nullptr,
+                                                int batch = 32) {
     constexpr int GPW = 32 / G;
     const int lane32 = threadIdx.x & 31;
     const int lane = threadIdx.x & (G - 1);
     const int gi = lane32 / G;
     const bool have_t = xt.ptr != nullptr;
-    {  // lane-parallel setup of the warp's next 32 LORs
+    {  // lane-parallel setup of the warp's next LORs
         const int64_t i = base + lane32;
         LeanRec E = {};
         E.lo = 1;
-        if (i < n) {
+        if (i < n && lane32 < batch) {
             const float *l = lors + i * stride;
             float lv[6];
 #pragma unroll
@@ -88,12 +110,12 @@ __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__r
             const float yv = y ? __ldg(y + i) : 1.0f;
             LorRec R = setup_rec<TOF>(lv, tv, yv, g, k);
             R.ad = add ? __ldg(add + i) : 0.0f;
-            E = make_lean<TOF>(R, g, k, x.st, xt.st, have_t);
+            E = make_lean<TOF, G>(R, g, k, x.st, xt.st, have_t, MODE == MODE_FUSED ? G * U : 0);
         }
         store_lean(&wrecs[lane32], E);
     }
     __syncwarp();
-    for (int j0 = 0; j0 < 32; j0 += GPW) {
+    for (int j0 = 0; j0 < batch; j0 += GPW) {
         const int j = j0 + gi;
         const LeanRec E = load_lean(&wrecs[j]);
         const int64_t i = base + j;
@@ -108,79 +130,70 @@ __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__r
             } else if (MODE == MODE_PROJ) {
                 const float p = tie_project<G, TOF>(lv, tv, lane, g, tp, x, xt);
                 if (lane == 0) out[i] = p;
+            } else if (MODE == MODE_ADJ) {
+                tie_backproject<G, TOF, RULES_PROJ>(lv, tv, E.yv, lane, g, tp, bp, bpt);
             } else {
-                tie_backproject<G, TOF>(lv, tv, E.yv, lane, g, tp, bp, bpt);
+                tie_backproject<G, TOF, RULES_BACK>(lv, tv, E.yv, lane, g, tp, bp, bpt);
             }
             continue;
         }
-        const bool valid = E.flags & F_VALID;
-        const bool xdom = E.flags & F_XDOM;
-        const LeanAxes ax = lean_axes(E, g, x.st, xt.st, have_t);
-        const float *xim = (!xdom && have_t) ? xt.ptr : x.ptr;
-        float *bim = (!xdom && have_t) ? bpt.ptr : bp.ptr;
-        // the projector's slabs: [plo, phi] (empty when the projector skips the LOR)
-        const int plo = (E.flags & F_PROJ) ? max(E.lo, E.pmlo) : 1;
-        const int phi = (E.flags & F_PROJ) ? min(E.hi, E.pmhi) : 0;
-        const bool shared = (plo == E.lo) && (phi == E.hi) && (E.hi - E.lo + 1 <= G * U);
-        int32_t o[U][3];
-        float w[U][3];
-        float acc = 0.0f;
-        if (MODE != MODE_BACK && valid) {
-            const float ppmax = (float)(phi - E.ic);
-            for (int c0 = plo; c0 <= phi; c0 += G * U) {
-                lean_chunk<TOF, U, G, QDIV>(E, ax, c0, phi, ppmax, lane, o, w);
-                float xv[U][3];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) xv[u][c] = (w[u][c] != 0.0f) ? __ldg(xim + o[u][c]) : 0.0f;
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) acc = fmaf(xv[u][c], w[u][c], acc);
-            }
-        }
-        float r;
-        if (MODE == MODE_BACK) {
-            if (!valid) continue;
-            r = E.yv;
-        } else {
+        const bool second = !(E.flags & F_XDOM) && have_t;
+        const float *xim = second ? xt.ptr : x.ptr;
+        float *bim = second ? bpt.ptr : bp.ptr;
+        const LeanAxes ax = lean_axes(E, g);
+        if (MODE == MODE_PROJ) {
+            float acc = 0.0f;
+            if (E.flags & F_VALID)
+                lean_walk<TOF, U, G, QDIV>(E, ax, E.plo, E.phi, lane, [&](auto &o, auto &w, auto ng) {
+                    acc = gather_slots<decltype(ng)::value>(xim, o, w, acc);
+                });
             const float p = group_sum<G>(acc) * E.invL2;
-            if (MODE == MODE_PROJ) {
-                if (lane == 0 && i < n) out[i] = p;  // 0 for a skipped LOR, as the reference's memset
-                continue;
+            if (lane == 0 && i < n) out[i] = p;  // 0 for a skipped LOR, as the reference's memset
+        } else if (MODE == MODE_BACK || MODE == MODE_ADJ) {
+            const float r = MODE == MODE_ADJ ? E.yv * E.invL2 : E.yv;
+            if (!(E.flags & F_VALID) || E.yv == 0.0f) continue;
+            const int lo = MODE == MODE_ADJ ? E.plo : E.lo, hi = MODE == MODE_ADJ ? E.phi : E.hi;
+            lean_walk<TOF, U, G, QDIV>(E, ax, lo, hi, lane, [&](auto &o, auto &w, auto ng) {
+                scatter_slots<decltype(ng)::value>(bim, o, w, r);
+            });
+        } else if (E.flags & F_HOT) {
+            static_assert(U == 2 || U == 4, "2 or 4 groups per chunk");
+            const int ng = E.flags >> kHotShift;
+            if (U > 2 && ng == 4) hot_lor<G, TOF, QDIV, U>(E, lane, xim, bim, rule, eps, ll, want_ll);
+            else if (U > 2 && ng == 3) hot_lor<G, TOF, QDIV, (U > 2 ? 3 : 1)>(E, lane, xim, bim, rule, eps, ll, want_ll);
+            else if (ng == 2) hot_lor<G, TOF, QDIV, 2>(E, lane, xim, bim, rule, eps, ll, want_ll);
+            else hot_lor<G, TOF, QDIV, 1>(E, lane, xim, bim, rule, eps, ll, want_ll);
+        } else if (E.flags & F_VALID) {
+            const bool shared = E.plo == E.lo && E.phi == E.hi && E.hi - E.lo < G * U;
+            int32_t o[U][3];
+            float w[U][3];
+            float acc = 0.0f;
+            if (shared) {
+                edge_chunk<TOF, U, G, QDIV>(E, ax, E.lo, E.hi, lane, o, w);
+                acc = gather_slots<U>(xim, o, w, 0.0f);
+            } else {
+                lean_walk<TOF, U, G, QDIV>(E, ax, E.plo, E.phi, lane, [&](auto &o_, auto &w_, auto ng) {
+                    acc = gather_slots<decltype(ng)::value>(xim, o_, w_, acc);
+                });
             }
-            if (!valid) continue;
+            const float p = group_sum<G>(acc) * E.invL2;
             const float den = __fadd_rn(__fadd_rn(p, E.ad), eps);
-            if (rule == SRF_RATIO_DIV_NO_NAN)
-                r = (den == 0.0f) ? 0.0f : __fdiv_rn(E.yv, den);
-            else
-                r = __fdiv_rn(E.yv, den);
+            const float r = ratio_of(E.yv, den, rule);
             if (want_ll && lane == 0 && den > 0.0f) ll += (double)E.yv * log((double)den);  // FP64 term and sum
-        }
-        if (r == 0.0f) continue;
-        if (MODE == MODE_FUSED && shared) {
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    if (w[u][c] != 0.0f) atomicAdd(bim + o[u][c], r * w[u][c]);
-        } else {
-            const float ppmax = (float)(E.hi - E.ic);
-            for (int c0 = E.lo; c0 <= E.hi; c0 += G * U) {
-                lean_chunk<TOF, U, G, QDIV>(E, ax, c0, E.hi, ppmax, lane, o, w);
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-                        if (w[u][c] != 0.0f) atomicAdd(bim + o[u][c], r * w[u][c]);
+            if (r == 0.0f) continue;
+            if (shared) {
+                scatter_slots<U>(bim, o, w, r);
+            } else {
+                lean_walk<TOF, U, G, QDIV>(E, ax, E.lo, E.hi, lane, [&](auto &o_, auto &w_, auto ng) {
+                    scatter_slots<decltype(ng)::value>(bim, o_, w_, r);
+                });
             }
         }
     }
     __syncwarp();
 }
 
-// One warp handles 32 consecutive LORs per round: lane j sets up LOR j into shared memory, then
+// One warp handles `batch` consecutive LORs per round (split_lors): lane j sets up LOR j into shared memory, then
 // the warp's 32/G groups walk the records. x/x_t and bp/bp_t have equal strides (offsets are
 // computed once for the gather and the scatter).
 // Single-study blocks are 128 threads: with the 4-slab variant's register budget (<= 102 per
@@ -192,7 +205,7 @@ __global__ void __launch_bounds__(kOsemBlock, MINB)
 k_osem_subset(const float *__restrict__ lors, int64_t n, int stride, const float *__restrict__ tof,
               int tof_stride, Grid g, TofParams tp, const float *__restrict__ y,
               const float *__restrict__ add, int rule, float eps, View x, View xt, View bp, View bpt,
-              double *__restrict__ loglik) {
+              double *__restrict__ loglik, int batch) {
     __shared__ LeanRec recs[kOsemBlock / 32][32];
     const int wib = threadIdx.x >> 5;
     const int lane32 = threadIdx.x & 31;
@@ -201,8 +214,8 @@ k_osem_subset(const float *__restrict__ lors, int64_t n, int stride, const float
     const GridK k = make_gridk<TOF>(g, tp);
     const bool want_ll = loglik != nullptr;
     double ll = 0.0;
-    for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
-        osem_warp_batch<G, TOF, U, MODE_FUSED, QDIV>(recs[wib], lors, n, stride, tof, tof_stride, g, k, tp, y, add, rule, eps, x, xt, bp, bpt, base, want_ll, ll);
+    for (int64_t base = warp * batch; base < n; base += nwarps * batch) {
+        osem_warp_batch<G, TOF, U, MODE_FUSED, QDIV>(recs[wib], lors, n, stride, tof, tof_stride, g, k, tp, y, add, rule, eps, x, xt, bp, bpt, base, want_ll, ll, nullptr, batch);
     }
     if (want_ll) {
 #pragma unroll
@@ -218,16 +231,16 @@ template <int G, bool TOF, int U, int MINB, int MODE, bool QDIV>
 __global__ void __launch_bounds__(kOsemBlock, MINB)
 k_trace_fused(const float *__restrict__ lors, int64_t n, int stride, const float *__restrict__ tof,
               int tof_stride, Grid g, TofParams tp, const float *__restrict__ values, float *__restrict__ out,
-              View v, View vt) {
+              View v, View vt, int batch) {
     __shared__ LeanRec recs[kOsemBlock / 32][32];
     const int wib = threadIdx.x >> 5;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const GridK k = make_gridk<TOF>(g, tp);
     double ll = 0.0;
-    for (int64_t base = warp * 32; base < n; base += nwarps * 32)
+    for (int64_t base = warp * batch; base < n; base += nwarps * batch)
         osem_warp_batch<G, TOF, U, MODE, QDIV>(recs[wib], lors, n, stride, tof, tof_stride, g, k, tp, values, nullptr,
-                                         SRF_RATIO_PLAIN, 0.0f, v, vt, v, vt, base, false, ll, out);
+                                         SRF_RATIO_PLAIN, 0.0f, v, vt, v, vt, base, false, ll, out, batch);
 }
 
 template <int G, bool TOF, int MODE>
@@ -235,8 +248,8 @@ static int launch_trace_fused_g(const float *lors, int64_t n, int stride, const 
                                 const Grid &g, const TofParams &tp, const float *values, float *out,
                                 const View &v, const View &vt, cudaStream_t s) {
     auto kern = grid_qdiv(g) ? k_trace_fused<G, TOF, 4, 5, MODE, true> : k_trace_fused<G, TOF, 4, 5, MODE, false>;
-    unsigned blocks = grid_for(kern, n, kOsemBlock, 0, kOsemBlock);
-    kern<<<blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, values, out, v, vt);
+    const LorSplit d = split_lors(kern, n, 32 / G, kOsemBlock);
+    kern<<<d.blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, values, out, v, vt, d.batch);
     return check_cuda("fused trace kernel launch");
 }
 
@@ -264,6 +277,12 @@ int fused_backprojection(const float *lors, int64_t n, int stride, const float *
                          const View &vt, cudaStream_t s) {
     return tof ? launch_trace_fused<true, MODE_BACK>(lors, n, stride, tof, tof_stride, g, tp, values, nullptr, v, vt, s)
                : launch_trace_fused<false, MODE_BACK>(lors, n, stride, nullptr, 1, g, tp, values, nullptr, v, vt, s);
+}
+
+int fused_adjoint(const float *lors, int64_t n, int stride, const float *tof, int tof_stride, const Grid &g,
+                  const TofParams &tp, const float *values, const View &v, const View &vt, cudaStream_t s) {
+    return tof ? launch_trace_fused<true, MODE_ADJ>(lors, n, stride, tof, tof_stride, g, tp, values, nullptr, v, vt, s)
+               : launch_trace_fused<false, MODE_ADJ>(lors, n, stride, nullptr, 1, g, tp, values, nullptr, v, vt, s);
 }
 
 // ---------------------------------------------------------------- sensitivity image
@@ -298,7 +317,7 @@ __device__ __forceinline__ void emap_warp(LeanRec *wrecs, const float *__restric
         if (i < n) {
             float lv[6];
             emap_endpoints(table, nb, m, i, lv);
-            E = make_lean<false>(setup_rec<false>(lv, 0.0f, 1.0f, g, k), g, k, v.st, vt.st, have_t);
+            E = make_lean<false, G>(setup_rec<false>(lv, 0.0f, 1.0f, g, k), g, k, v.st, vt.st, have_t, 0);
         }
         store_lean(&wrecs[lane32], E);
     }
@@ -310,23 +329,14 @@ __device__ __forceinline__ void emap_warp(LeanRec *wrecs, const float *__restric
         if (E.flags & F_TIE) {  // the backprojector's own axis differs from the projector's: generic path
             float lv[6];
             emap_endpoints(table, nb, m, i, lv);
-            tie_backproject<G, false>(lv, 0.0f, 1.0f, lane, g, tp, v, vt);
+            tie_backproject<G, false, RULES_BACK>(lv, 0.0f, 1.0f, lane, g, tp, v, vt);
             continue;
         }
         if (!(E.flags & F_VALID)) continue;
-        const LeanAxes ax = lean_axes(E, g, v.st, vt.st, have_t);
         float *im = (!(E.flags & F_XDOM) && have_t) ? vt.ptr : v.ptr;
-        int32_t o[U][3];
-        float w[U][3];
-        const float ppmax = (float)(E.hi - E.ic);
-        for (int c0 = E.lo; c0 <= E.hi; c0 += G * U) {
-            lean_chunk<false, U, G, QDIV>(E, ax, c0, E.hi, ppmax, lane, o, w);
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    if (w[u][c] != 0.0f) atomicAdd(im + o[u][c], w[u][c]);
-        }
+        lean_walk<false, U, G, QDIV>(E, lean_axes(E, g), E.lo, E.hi, lane, [&](auto &o, auto &w, auto ng) {
+            scatter_slots<decltype(ng)::value>(im, o, w, 1.0f);
+        });
     }
     __syncwarp();
 }
@@ -386,7 +396,7 @@ __device__ __forceinline__ void batch_warp(LeanRec *wrecs, const float *__restri
                                            const float *__restrict__ tof, int tof_stride, const Grid &g,
                                            const GridK &k, const TofParams &tp, int nb, int64_t bstride,
                                            const float *__restrict__ values, float *__restrict__ out,
-                                           int64_t ostride, const View &v, const View &vt, int64_t base) {
+                                           int64_t ostride, const View &v, const View &vt, int64_t base, int batch) {
     constexpr int GPW = 32 / G;
     const int lane32 = threadIdx.x & 31;
     const int lane = threadIdx.x & (G - 1);
@@ -396,18 +406,18 @@ __device__ __forceinline__ void batch_warp(LeanRec *wrecs, const float *__restri
         const int64_t i = base + lane32;
         LeanRec E = {};
         E.lo = 1;
-        if (i < n) {
+        if (i < n && lane32 < batch) {
             const float *l = lors + i * stride;
             float lv[6];
 #pragma unroll
             for (int c = 0; c < 6; ++c) lv[c] = __ldg(l + c);
             const float tv = TOF ? __ldg(tof + i * tof_stride) : 0.0f;
-            E = make_lean<TOF>(setup_rec<TOF>(lv, tv, 1.0f, g, k), g, k, v.st, vt.st, have_t);
+            E = make_lean<TOF, G>(setup_rec<TOF>(lv, tv, 1.0f, g, k), g, k, v.st, vt.st, have_t, 0);
         }
         store_lean(&wrecs[lane32], E);
     }
     __syncwarp();
-    for (int j0 = 0; j0 < 32; j0 += GPW) {
+    for (int j0 = 0; j0 < batch; j0 += GPW) {
         const int j = j0 + gi;
         const LeanRec E = load_lean(&wrecs[j]);
         const int64_t i = base + j;
@@ -426,20 +436,13 @@ __device__ __forceinline__ void batch_warp(LeanRec *wrecs, const float *__restri
             for (int c = 0; c < 6; ++c) lv[c] = __ldg(l + c);
             if (MODE == MODE_PROJ || any) tie_batch<G, TOF, MODE>(lv, 0.0f, lane, g, tp, v, vt, nb, bstride, val, acc);
         } else if ((E.flags & F_VALID) && (E.flags & F_PROJ) && (MODE == MODE_PROJ || any)) {
-            const LeanAxes ax = lean_axes(E, g, v.st, vt.st, have_t);
             float *im = (!(E.flags & F_XDOM) && have_t) ? vt.ptr : v.ptr;
             if (MODE == MODE_ADJ)
 #pragma unroll
                 for (int b = 0; b < kMaxBatch; ++b) val[b] *= E.invL2;
-            // the projector's slabs: its endpoint rule keeps [pmlo, pmhi]
-            const int plo = max(E.lo, E.pmlo), phi = min(E.hi, E.pmhi);
-            const float ppmax = (float)(phi - E.ic);
-            int32_t o[U][3];
-            float w[U][3];
-            for (int c0 = plo; c0 <= phi; c0 += G * U) {
-                lean_chunk<TOF, U, G, QDIV>(E, ax, c0, phi, ppmax, lane, o, w);
+            lean_walk<TOF, U, G, QDIV>(E, lean_axes(E, g), E.plo, E.phi, lane, [&](auto &o, auto &w, auto ng) {
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                for (int u = 0; u < decltype(ng)::value; ++u)
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         if (w[u][c] == 0.0f) continue;
@@ -450,7 +453,7 @@ __device__ __forceinline__ void batch_warp(LeanRec *wrecs, const float *__restri
                             else if (val[b] != 0.0f) atomicAdd(im + b * bstride + o[u][c], val[b] * w[u][c]);
                         }
                     }
-            }
+            });
 #pragma unroll
             for (int b = 0; b < kMaxBatch; ++b) acc[b] *= E.invL2;
         }
@@ -469,15 +472,16 @@ template <int G, bool TOF, int U, int MINB, int MODE, bool QDIV>
 __global__ void __launch_bounds__(kOsemBlock, MINB)
 k_trace_fused_batch(const float *__restrict__ lors, int64_t n, int stride, const float *__restrict__ tof,
                     int tof_stride, Grid g, TofParams tp, int nb, int64_t bstride,
-                    const float *__restrict__ values, float *__restrict__ out, int64_t ostride, View v, View vt) {
+                    const float *__restrict__ values, float *__restrict__ out, int64_t ostride, View v, View vt,
+                    int batch) {
     __shared__ LeanRec recs[kOsemBlock / 32][32];
     const int wib = threadIdx.x >> 5;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const GridK k = make_gridk<TOF>(g, tp);
-    for (int64_t base = warp * 32; base < n; base += nwarps * 32)
+    for (int64_t base = warp * batch; base < n; base += nwarps * batch)
         batch_warp<G, TOF, U, MODE, QDIV>(recs[wib], lors, n, stride, tof, tof_stride, g, k, tp, nb, bstride, values,
-                                          out, ostride, v, vt, base);
+                                          out, ostride, v, vt, base, batch);
 }
 
 template <bool TOF, int MODE>
@@ -486,8 +490,8 @@ static int launch_fused_batch(const float *lors, int64_t n, int stride, const fl
                               float *out, int64_t ostride, const View &v, const View &vt, cudaStream_t s) {
     if (n == 0) return ok();
     auto kern = grid_qdiv(g) ? k_trace_fused_batch<32, TOF, 4, 4, MODE, true> : k_trace_fused_batch<32, TOF, 4, 4, MODE, false>;
-    unsigned blocks = grid_for(kern, n, kOsemBlock, 0, kOsemBlock);
-    kern<<<blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, nb, bstride, values, out, ostride, v, vt);
+    const LorSplit d = split_lors(kern, n, 1, kOsemBlock);
+    kern<<<d.blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, nb, bstride, values, out, ostride, v, vt, d.batch);
     return check_cuda("batched projector kernel launch");
 }
 
@@ -511,8 +515,8 @@ static int launch_osem_g(const float *lors, int64_t n, int stride, const float *
                          const View &x, const View &xt, const View &bp, const View &bpt,
                          double *loglik, cudaStream_t s) {
     auto kern = grid_qdiv(g) ? k_osem_subset<G, TOF, U, MINB, true> : k_osem_subset<G, TOF, U, MINB, false>;
-    unsigned blocks = grid_for(kern, n, kOsemBlock, 0, kOsemBlock);
-    kern<<<blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, y, add, rule, eps, x, xt, bp, bpt, loglik);
+    const LorSplit d = split_lors(kern, n, 32 / G, kOsemBlock);
+    kern<<<d.blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, y, add, rule, eps, x, xt, bp, bpt, loglik, d.batch);
     return check_cuda("osem subset kernel launch");
 }
 
