@@ -425,7 +425,7 @@ __device__ __forceinline__ void edge_chunk(const LeanRec &E, const LeanAxes &ax,
     }
 }
 
-// Sum of im * w over the slots of N groups; im += r * w over them.
+// Sum of im * w over the slots of N groups.
 template <int N>
 __device__ __forceinline__ float gather_slots(const float *__restrict__ im, const int32_t (*o)[3], const float (*w)[3], float acc) {
     float x[N][3];
@@ -440,13 +440,26 @@ __device__ __forceinline__ float gather_slots(const float *__restrict__ im, cons
     return acc;
 }
 
-template <int N>
-__device__ __forceinline__ void scatter_slots(float *im, const int32_t (*o)[3], const float (*w)[3], float r) {
+// Slots 0 and 1 of a group's G slabs go out as two accesses of G lanes, the first with both slots of the
+// lower G / 2 slabs, the second with those of the upper ones: the slab after an in-plane crossing continues
+// the row that the crossing slab's slot 1 begins, so that one instruction carries both into one
+// 32-byte sector. As separate slot 0 and slot 1 accesses the L2's reduction sectors were the bound (181 M
+// per 2e6 TOF LORs, 1.0 ms at the rate of coalesced ones): non-TOF backprojection of 2e6 LORs
+// 2,136 -> 1,422 us. Gathers are not dealt anew: projection alone was 6 % slower with the two shuffles.
+template <int G, int N>
+__device__ __forceinline__ void scatter_slots(float *im, const int32_t (*o)[3], const float (*w)[3], float r, int lane) {
+    const bool upper = lane & (G / 2);
+    const unsigned m = group_mask<G>();
 #pragma unroll
-    for (int u = 0; u < N; ++u)
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            if (w[u][c] != 0.0f) atomicAdd(im + o[u][c], r * w[u][c]);
+    for (int u = 0; u < N; ++u) {
+        const float r0 = r * w[u][0], r1 = r * w[u][1];
+        const int32_t ox = __shfl_xor_sync(m, o[u][1], G / 2, G);
+        const float rx = __shfl_xor_sync(m, r1, G / 2, G);
+        const float ra = upper ? rx : r0, rb = upper ? r0 : rx;
+        if (ra != 0.0f) atomicAdd(im + (upper ? ox : o[u][0]), ra);
+        if (rb != 0.0f) atomicAdd(im + (upper ? o[u][0] : ox), rb);
+        if (w[u][2] != 0.0f) atomicAdd(im + o[u][2], r * w[u][2]);
+    }
 }
 
 }  // namespace srf

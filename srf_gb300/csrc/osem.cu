@@ -61,19 +61,21 @@ __device__ __forceinline__ float ratio_of(float yv, float den, int rule) {
     return __fdiv_rn(yv, den);
 }
 
-// The fused step of a LOR whose N groups are all interior (F_HOT): one straight line from the slabs'
-// arithmetic over the gathers and the ratio to the reductions.
-template <int G, bool TOF, bool QDIV, int N>
-__device__ __forceinline__ void hot_lor(const LeanRec &E, int lane, const float *xim, float *bim, int rule, float eps,
-                                        double &ll, bool want_ll) {
+// The fused step of a LOR of N groups (one chunk): one straight line from the slabs' arithmetic over the
+// gathers and the ratio to the reductions. EDGE: groups with range tests (short LORs that reach the image
+// faces), else all groups are interior (F_HOT).
+template <int G, bool TOF, bool QDIV, int N, bool EDGE>
+__device__ __forceinline__ void chunk_lor(const LeanRec &E, const LeanAxes &ax, int lane, const float *xim, float *bim, int rule,
+                                          float eps, double &ll, bool want_ll) {
     int32_t o[N][3];
     float w[N][3];
-    interior_groups<TOF, G, QDIV, N>(E, E.lo, E.hi, lane, o, w);
+    if (EDGE) edge_chunk<TOF, N, G, QDIV>(E, ax, E.lo, E.hi, lane, o, w);
+    else interior_groups<TOF, G, QDIV, N>(E, E.lo, E.hi, lane, o, w);
     const float p = group_sum<G>(gather_slots<N>(xim, o, w, 0.0f)) * E.invL2;
     const float den = __fadd_rn(__fadd_rn(p, E.ad), eps);
     const float r = ratio_of(E.yv, den, rule);
     if (want_ll && lane == 0 && den > 0.0f) ll += (double)E.yv * log((double)den);  // FP64 term and sum
-    if (r != 0.0f) scatter_slots<N>(bim, o, w, r);
+    if (r != 0.0f) scatter_slots<G, N>(bim, o, w, r, lane);  // r is the group's
 }
 
 // LORs [base, base + batch) of one study (batch <= 32, a multiple of 32 / G): lane-parallel setup of
@@ -154,40 +156,33 @@ __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__r
             if (!(E.flags & F_VALID) || E.yv == 0.0f) continue;
             const int lo = MODE == MODE_ADJ ? E.plo : E.lo, hi = MODE == MODE_ADJ ? E.phi : E.hi;
             lean_walk<TOF, U, G, QDIV>(E, ax, lo, hi, lane, [&](auto &o, auto &w, auto ng) {
-                scatter_slots<decltype(ng)::value>(bim, o, w, r);
+                scatter_slots<G, decltype(ng)::value>(bim, o, w, r, lane);
             });
         } else if (E.flags & F_HOT) {
             static_assert(U == 2 || U == 4, "2 or 4 groups per chunk");
             const int ng = E.flags >> kHotShift;
-            if (U > 2 && ng == 4) hot_lor<G, TOF, QDIV, U>(E, lane, xim, bim, rule, eps, ll, want_ll);
-            else if (U > 2 && ng == 3) hot_lor<G, TOF, QDIV, (U > 2 ? 3 : 1)>(E, lane, xim, bim, rule, eps, ll, want_ll);
-            else if (ng == 2) hot_lor<G, TOF, QDIV, 2>(E, lane, xim, bim, rule, eps, ll, want_ll);
-            else hot_lor<G, TOF, QDIV, 1>(E, lane, xim, bim, rule, eps, ll, want_ll);
+            if (U > 2 && ng == 4) chunk_lor<G, TOF, QDIV, U, false>(E, ax, lane, xim, bim, rule, eps, ll, want_ll);
+            else if (U > 2 && ng == 3) chunk_lor<G, TOF, QDIV, (U > 2 ? 3 : 1), false>(E, ax, lane, xim, bim, rule, eps, ll, want_ll);
+            else if (ng == 2) chunk_lor<G, TOF, QDIV, 2, false>(E, ax, lane, xim, bim, rule, eps, ll, want_ll);
+            else chunk_lor<G, TOF, QDIV, 1, false>(E, ax, lane, xim, bim, rule, eps, ll, want_ll);
         } else if (E.flags & F_VALID) {
-            const bool shared = E.plo == E.lo && E.phi == E.hi && E.hi - E.lo < G * U;
-            int32_t o[U][3];
-            float w[U][3];
-            float acc = 0.0f;
-            if (shared) {
-                edge_chunk<TOF, U, G, QDIV>(E, ax, E.lo, E.hi, lane, o, w);
-                acc = gather_slots<U>(xim, o, w, 0.0f);
-            } else {
-                lean_walk<TOF, U, G, QDIV>(E, ax, E.plo, E.phi, lane, [&](auto &o_, auto &w_, auto ng) {
-                    acc = gather_slots<decltype(ng)::value>(xim, o_, w_, acc);
-                });
+            if (E.plo == E.lo && E.phi == E.hi && E.hi - E.lo < 2 * G) {
+                chunk_lor<G, TOF, QDIV, 2, true>(E, ax, lane, xim, bim, rule, eps, ll, want_ll);
+                continue;
             }
+            // a long LOR, or one that the projector's endpoint rule cuts: two walks
+            float acc = 0.0f;
+            lean_walk<TOF, 2, G, QDIV>(E, ax, E.plo, E.phi, lane, [&](auto &o_, auto &w_, auto ng) {
+                acc = gather_slots<decltype(ng)::value>(xim, o_, w_, acc);
+            });
             const float p = group_sum<G>(acc) * E.invL2;
             const float den = __fadd_rn(__fadd_rn(p, E.ad), eps);
             const float r = ratio_of(E.yv, den, rule);
             if (want_ll && lane == 0 && den > 0.0f) ll += (double)E.yv * log((double)den);  // FP64 term and sum
             if (r == 0.0f) continue;
-            if (shared) {
-                scatter_slots<U>(bim, o, w, r);
-            } else {
-                lean_walk<TOF, U, G, QDIV>(E, ax, E.lo, E.hi, lane, [&](auto &o_, auto &w_, auto ng) {
-                    scatter_slots<decltype(ng)::value>(bim, o_, w_, r);
-                });
-            }
+            lean_walk<TOF, 2, G, QDIV>(E, ax, E.lo, E.hi, lane, [&](auto &o_, auto &w_, auto ng) {
+                scatter_slots<G, decltype(ng)::value>(bim, o_, w_, r, lane);
+            });
         }
     }
     __syncwarp();
@@ -196,8 +191,11 @@ __device__ __forceinline__ void osem_warp_batch(LeanRec *wrecs, const float *__r
 // One warp handles `batch` consecutive LORs per round (split_lors): lane j sets up LOR j into shared memory, then
 // the warp's 32/G groups walk the records. x/x_t and bp/bp_t have equal strides (offsets are
 // computed once for the gather and the scatter).
-// Single-study blocks are 128 threads: with the 4-slab variant's register budget (<= 102 per
-// thread at 5 blocks per SM) that is 20 resident warps per SM instead of 16 with 256-thread blocks.
+// Single-study blocks are 128 threads. The fused step runs 6 per SM (80 registers, 24 warps), the
+// projector and backprojector 7 (72): 2e6 TOF LORs 1.03 ms with 5, 6 or 7 blocks, 1e5 LORs on the
+// smaller grids 50-58 us; projection 1.31 ms (5) against 1.22 ms (7). What sets these kernels' time besides
+// L2 is the instruction cache: with the range-tested chunk of a short LOR unrolled over four groups
+// and walks of up to four, the fused kernel was 9 % slower at clinical size and 27 % on small grids.
 constexpr int kOsemBlock = 128;
 
 template <int G, bool TOF, int U, int MINB, bool QDIV>
@@ -247,7 +245,7 @@ template <int G, bool TOF, int MODE>
 static int launch_trace_fused_g(const float *lors, int64_t n, int stride, const float *tof, int tof_stride,
                                 const Grid &g, const TofParams &tp, const float *values, float *out,
                                 const View &v, const View &vt, cudaStream_t s) {
-    auto kern = grid_qdiv(g) ? k_trace_fused<G, TOF, 4, 5, MODE, true> : k_trace_fused<G, TOF, 4, 5, MODE, false>;
+    auto kern = grid_qdiv(g) ? k_trace_fused<G, TOF, 4, 7, MODE, true> : k_trace_fused<G, TOF, 4, 7, MODE, false>;
     const LorSplit d = split_lors(kern, n, 32 / G, kOsemBlock);
     kern<<<d.blocks, kOsemBlock, 0, s>>>(lors, n, stride, tof, tof_stride, g, tp, values, out, v, vt, d.batch);
     return check_cuda("fused trace kernel launch");
@@ -335,7 +333,7 @@ __device__ __forceinline__ void emap_warp(LeanRec *wrecs, const float *__restric
         if (!(E.flags & F_VALID)) continue;
         float *im = (!(E.flags & F_XDOM) && have_t) ? vt.ptr : v.ptr;
         lean_walk<false, U, G, QDIV>(E, lean_axes(E, g), E.lo, E.hi, lane, [&](auto &o, auto &w, auto ng) {
-            scatter_slots<decltype(ng)::value>(im, o, w, 1.0f);
+            scatter_slots<G, decltype(ng)::value>(im, o, w, 1.0f, lane);
         });
     }
     __syncwarp();
@@ -527,7 +525,7 @@ static int launch_osem_u(const float *lors, int64_t n, int stride, const float *
                          double *loglik, cudaStream_t s) {
     if (slabs_per_lane() == 2)
         return launch_osem_g<G, TOF, 2, 6>(lors, n, stride, tof, tof_stride, g, tp, y, add, rule, eps, x, xt, bp, bpt, loglik, s);
-    return launch_osem_g<G, TOF, 4, 5>(lors, n, stride, tof, tof_stride, g, tp, y, add, rule, eps, x, xt, bp, bpt, loglik, s);
+    return launch_osem_g<G, TOF, 4, 6>(lors, n, stride, tof, tof_stride, g, tp, y, add, rule, eps, x, xt, bp, bpt, loglik, s);
 }
 
 template <bool TOF>
