@@ -185,6 +185,12 @@ int srf_fold_views(float *dst, const int64_t dst_strides[3], const float *src,
 int srf_copy_view(float *dst, const int64_t dst_strides[3], const float *src,
                   const int64_t src_strides[3], const int32_t grid[3], void *stream);
 
+/* dst = src (+ src2) and dst2 = the same, for images of one grid with strides of their own (elements);
+ * src2 and dst2 may be NULL. No destination may overlap a source. */
+int srf_relayout(const float *src, const int64_t src_strides[3], const float *src2,
+                 const int64_t src2_strides[3], float *dst, const int64_t dst_strides[3], float *dst2,
+                 const int64_t dst2_strides[3], const int32_t grid[3], void *stream);
+
 /* ------------------------------------------------------------------ MLEM / OSEM */
 
 /* Ratio rules of the reference's update loops:

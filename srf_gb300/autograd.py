@@ -43,7 +43,7 @@ class _Project(torch.autograd.Function):
 
         if dim == 3:
             grad = kernels.backproject(lors, g.contiguous(), shape, center, size, tof=tof,
-                                       tof_nsigma=tof_nsigma, adjoint=True)
+                                       tof_nsigma=tof_nsigma, adjoint=True, order="z")
         else:
             B = kernels.MAX_BATCH
             grad = _joined([kernels.adjoint_batch(lors, g[k:k + B], shape, center, size, tof=tof,

@@ -46,7 +46,7 @@ class EcatEmapGenerator(_NefLike):
         else:
             raise NotImplementedError(f"emap mode {self.mode!r}")
         t = torch.as_tensor(table, dtype=torch.float32).to(device())
-        acc = kernels.emap_block_full(t, nb, shape, center, size).contiguous()
+        acc = kernels.emap_block_full(t, nb, shape, center, size, order="z")
         ref = getattr(image, "data", None)
         return Emap(like_input(acc, ref if ref is not None else np.zeros(0), "tf-eager"),
                     center, size)

@@ -109,8 +109,8 @@ class BackProject(_NefLike):
         _mode_ok(self.mode)
         shape, center, size = _geom(image)
         bp = kernels.backproject(_lors_dev(listmode.lors, False), to_dev(listmode.data), shape,
-                                 center, size)
-        return image.update(data=like_input(bp.contiguous(), image.data, self.mode))
+                                 center, size, order="z")
+        return image.update(data=like_input(bp, image.data, self.mode))
 
 
 @dataclasses.dataclass(frozen=True)
@@ -138,5 +138,5 @@ class BackProjectTof(_NefLike):
         shape, center, size = _geom(image)
         bp = kernels.backproject(_lors_dev(listmode.lors, True), to_dev(listmode.data), shape,
                                  center, size, tof=(self.tof.tof_bin, self.tof.tof_sigma2),
-                                 tof_nsigma=self.tof_nsigma)
-        return image.update(data=like_input(bp.contiguous(), image.data, self.mode))
+                                 tof_nsigma=self.tof_nsigma, order="z")
+        return image.update(data=like_input(bp, image.data, self.mode))

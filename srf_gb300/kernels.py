@@ -58,6 +58,47 @@ def new_yfast(shape: Sequence[int], device) -> torch.Tensor:
     return torch.zeros((nz, nx, ny), dtype=F32, device=device).permute(1, 2, 0)
 
 
+def _relayout(shape, src: torch.Tensor, src2: Optional[torch.Tensor], dst: torch.Tensor,
+              dst2: Optional[torch.Tensor] = None) -> None:
+    """dst = src (+ src2), and dst2 the same: (nx, ny, nz) views of any strides, one pass."""
+    st = lambda t: None if t is None else i64x3(t.stride())
+    call("srf_relayout", ptr(src), st(src), ptr(src2), st(src2), ptr(dst), st(dst), ptr(dst2), st(dst2), i32x3(shape),
+         stream_ptr(src.device))
+
+
+def _empty_layout(shape, order: str, device) -> torch.Tensor:
+    """Uninitialised (nx, ny, nz) view whose memory is x-, y- or z-fastest."""
+    nx, ny, nz = shape
+    if order == "x":
+        return torch.empty((nz, ny, nx), dtype=F32, device=device).permute(2, 1, 0)
+    if order == "y":
+        return torch.empty((nz, nx, ny), dtype=F32, device=device).permute(1, 2, 0)
+    return torch.empty((nx, ny, nz), dtype=F32, device=device)
+
+
+def _projector_layouts(image: torch.Tensor, want_t: bool):
+    """The x-fastest image (the image itself when it is) and, when wanted, its y-fastest copy."""
+    shape = list(image.shape)
+    have_x = image.stride(0) == 1
+    if sum((n - 1) * s for n, s in zip(shape, image.stride())) >= 1 << 31:  # a view far beyond its own voxels
+        image = image if have_x else xfast(image)
+        return image, yfast(image) if want_t else None
+    x = image if have_x else _empty_layout(shape, "x", image.device)
+    t = _empty_layout(shape, "y", image.device) if want_t else None
+    if not have_x:
+        _relayout(shape, image, None, x, t)
+    elif want_t:
+        _relayout(shape, image, None, t)
+    return x, t
+
+
+def _accumulators(shape, device):
+    """Zeroed x-fastest and y-fastest accumulators of one image."""
+    nx, ny, nz = shape
+    acc = torch.zeros((2, nz, ny * nx), dtype=F32, device=device)
+    return acc[0].view(nz, ny, nx).permute(2, 1, 0), acc[1].view(nz, nx, ny).permute(1, 2, 0)
+
+
 def _tof_args(tof_bin, tof_sigma2, nsigma):
     return f32(tof_bin), f32(tof_sigma2), f32(nsigma)
 
@@ -69,10 +110,10 @@ def project(lors: torch.Tensor, image: torch.Tensor, center, size, *, tof: Optio
     n, stride = check_lors(lors, tof is not None)
     _require_cuda(image, "image")
     shape = list(image.shape)
-    if image.stride(0) != 1:
-        image = xfast(image)
-    if image_t is None and make_t:
-        image_t = yfast(image)
+    if image.dim() != 3:
+        raise ValueError("image must be (nx, ny, nz)")
+    image, made_t = _projector_layouts(image, image_t is None and make_t)
+    image_t = made_t if image_t is None else image_t
     if out is None:
         out = torch.empty(n, dtype=F32, device=lors.device)
     st = i64x3(image.stride())
@@ -90,16 +131,16 @@ def project(lors: torch.Tensor, image: torch.Tensor, center, size, *, tof: Optio
 
 def backproject(lors: torch.Tensor, values: torch.Tensor, shape, center, size, *,
                 tof: Optional[Tuple[float, float]] = None, tof_nsigma: float = 0.0,
-                adjoint: bool = False, use_t: bool = True) -> torch.Tensor:
-    """A_bp^T values as an x-fastest (nx, ny, nz) tensor (adjoint=True: exact adjoint of
-    ``project``)."""
+                adjoint: bool = False, use_t: bool = True, order: str = "x") -> torch.Tensor:
+    """A_bp^T values as an x-fastest (nx, ny, nz) tensor (order 'z': a contiguous one; adjoint=True:
+    exact adjoint of ``project``)."""
     n, stride = check_lors(lors, tof is not None)
     _require_cuda(values, "values")
     values = values.contiguous()
     if values.numel() != n:
         raise ValueError("values must have one entry per LOR")
-    acc = new_xfast(shape, lors.device)
-    acc_t = new_yfast(shape, lors.device) if use_t else None
+    shape = list(shape)
+    acc, acc_t = _accumulators(shape, lors.device) if use_t else (new_xfast(shape, lors.device), None)
     st = i64x3(acc.stride())
     t_args = (ptr(acc_t), i64x3(acc_t.stride())) if acc_t is not None else (None, None)
     s = stream_ptr(lors.device)
@@ -116,9 +157,16 @@ def backproject(lors: torch.Tensor, values: torch.Tensor, shape, center, size, *
         call("srf_backprojection_tof", ptr(lors), i64(n), i32(stride), _tof_ptr(lors), i32(stride),
              *_tof_args(tof[0], tof[1], tof_nsigma), ptr(values), ptr(acc), st, *t_args,
              i32x3(shape), f32x3(center), f32x3(size), s)
-    if acc_t is not None:
-        fold(acc, acc_t)
-    return acc
+    return _folded(shape, acc, acc_t, order)
+
+
+def _folded(shape, acc: torch.Tensor, acc_t: Optional[torch.Tensor], order: str) -> torch.Tensor:
+    """The two accumulators as one image."""
+    if acc_t is None and order == "x":
+        return acc
+    out = _empty_layout(shape, order, acc.device)
+    _relayout(shape, acc, acc_t, out)
+    return out
 
 
 MAX_BATCH = 8
@@ -238,19 +286,27 @@ class SubsetState:
 
     def __init__(self, shape, center, size, device, x0: Optional[torch.Tensor] = None):
         self.shape, self.center, self.size = list(shape), list(center), list(size)
-        self.x = new_xfast(shape, device)
-        if x0 is None:
-            self.x.fill_(1.0)
-        else:
-            self.x.copy_(x0)
-        self.x_t = yfast(self.x)
-        # both backprojection accumulators in one flat buffer (one collective sums both)
         nx, ny, nz = self.shape
+        if x0 is None:
+            one = torch.ones((2, nz, ny * nx), dtype=F32, device=device)
+            self.x = one[0].view(nz, ny, nx).permute(2, 1, 0)
+            self.x_t = one[1].view(nz, nx, ny).permute(1, 2, 0)
+        else:
+            self.x = new_xfast(shape, device)
+            self.x.copy_(x0)
+            self.x_t = yfast(self.x)
+        # both backprojection accumulators in one flat buffer (one collective sums both)
         v = nx * ny * nz
         self._acc = torch.zeros(2 * v, dtype=F32, device=device)
         self.bp = self._acc[:v].view(nz, ny, nx).permute(2, 1, 0)
         self.bp_t = self._acc[v:].view(nz, nx, ny).permute(1, 2, 0)
         self.loglik = torch.zeros(1, dtype=torch.float64, device=device)
+
+    def image(self) -> torch.Tensor:
+        """A contiguous (nx, ny, nz) copy of x."""
+        out = _empty_layout(self.shape, "z", self.x.device)
+        _relayout(self.shape, self.x, None, out)
+        return out
 
     def accumulators(self) -> torch.Tensor:
         """The flat buffer holding both backprojection accumulators (what an event-sharded
@@ -277,18 +333,17 @@ class SubsetState:
              stream_ptr(self.x.device))
 
 
-def emap_block_full(table: torch.Tensor, n_blocks: int, shape, center, size) -> torch.Tensor:
+def emap_block_full(table: torch.Tensor, n_blocks: int, shape, center, size, order: str = "x") -> torch.Tensor:
     _require_cuda(table, "crystal table")
     m = table.shape[0] // n_blocks
-    acc = new_xfast(shape, table.device)
-    acc_t = new_yfast(shape, table.device)
+    shape = list(shape)
+    acc, acc_t = _accumulators(shape, table.device)
     need = int(_lib.load().srf_emap_workspace(i32(n_blocks), i32(m)))
     ws = torch.empty(need, dtype=torch.uint8, device=table.device) if need else None
     call("srf_emap_block_full_ws", ptr(table), i32(n_blocks), i32(m), ptr(acc), i64x3(acc.stride()),
          ptr(acc_t), i64x3(acc_t.stride()), i32x3(shape), f32x3(center), f32x3(size), ptr(ws), i64(need),
          stream_ptr(table.device))
-    fold(acc, acc_t)
-    return acc
+    return _folded(shape, acc, acc_t, order)
 
 
 def sss(pairs: torch.Tensor, crystal_pos: torch.Tensor, scatter_pos: torch.Tensor,

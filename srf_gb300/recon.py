@@ -68,7 +68,7 @@ def _emap_dev(emap) -> torch.Tensor:
 
 
 def _result(state: kernels.SubsetState, like, center, size) -> Image:
-    x = state.x.contiguous()
+    x = state.image()
     if not isinstance(like, torch.Tensor):
         x = x.cpu().numpy()
     return Image(x, list(center), list(size))
