@@ -33,9 +33,9 @@ constexpr int F_VALID = 1, F_PROJ = 2, F_XDOM = 4, F_TIE = 8;
 
 // a / b rounded to nearest from rb = RN(1 / b): two Newton steps on residuals that the FMA computes
 // exactly (Markstein's division). Five instructions where the setup's divisions share a divisor (the
-// voxel size, the slab axis extent, the LOR length) instead of about ten and a branch each. Operands
-// far from the ends of the exponent range; where a is infinite the quotient is NaN, which the finite
-// tests and comparisons that follow treat alike.
+// voxel size, the slab axis extent, the LOR length) instead of about ten and a branch each. Operands far
+// from the ends of the exponent range. Where the quotient overflows this gives NaN instead of infinity: the
+// finite tests and comparisons that follow treat both alike, and make_lean sets an overflowed TOF value right.
 __device__ __forceinline__ float div_exact(float a, float b, float rb) {
     float q = __fmul_rn(a, rb);
     q = __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);

@@ -175,7 +175,9 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
         const float pc = __fmul_rn(__fadd_rn((float)(ic - np_half), 0.5f), dpc);
         const float dic = __fmul_rn(__fsub_rn(div_exact(__fsub_rn(pc, R.p1), R.pd, R.rpd), R.ratio1), R.L);
         E.tS = tA * s;
-        E.tT = dic * s;
+        // NaN: a finite TOF value whose quotient by the voxel size overflowed (infinite in IEEE division); it lies
+        // infinitely far from every slab
+        E.tT = dic == dic ? dic * s : INFINITY;
     }
     // interior slabs: both faces of every slab within the box by the margin, in q and in z
     float qa, qb, za, zb;
