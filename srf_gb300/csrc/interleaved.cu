@@ -7,9 +7,11 @@
 // What bounds the separate-image form is its accesses: per slab and slot a warp touches ~11 sectors
 // of 32 bytes in each image (32 slabs cross ~14 rows of 8 voxels), 91 for eight images, in eight
 // instructions. Interleaved by eight, a voxel is one sector whatever the direction of the LOR: 32
-// sectors in two instructions, and no second layout for y-dominant LORs (W = 2 and 4 keep one).
+// sectors in two instructions, and projections need no second layout for y-dominant LORs (W = 2 and 4
+// keep one). Adjoints keep a second accumulator at every width: with one, a voxel's sum has twice the rms
+// rounding error (1.97 times at 1,100 terms a voxel).
 // Measured, 8 images 128 x 128 x 64, 5e6 TOF LORs at 3 sigma, projection + adjoint with the loss between
-// them: 21.7 -> 8.0 ms.
+// them: 21.7 -> 7.6 ms (8.0 ms with one accumulator).
 #include "common.cuh"
 #include "fused.cuh"
 #include "lean.cuh"

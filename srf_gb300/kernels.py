@@ -180,12 +180,13 @@ def _width(B: int, shape) -> int:
 
 
 def _interleaved(shape, width: int, device, fill: bool):
-    """Interleaved buffers: x-fastest, and y-fastest for the y-dominant LORs where a voxel is less than a
-    32-byte sector."""
+    """Interleaved buffers: x-fastest, and y-fastest for the y-dominant LORs. Images to read need the second one
+    only where a voxel is less than a 32-byte sector; accumulators (fill) always have both: one sum over
+    both kinds of LORs would round twice as much (rms) as the two."""
     nx, ny, nz = shape
     new = torch.zeros if fill else torch.empty
     il = new((nz, ny, nx, width), dtype=F32, device=device)
-    return il, (new((nz, nx, ny, width), dtype=F32, device=device) if width < 8 else None)
+    return il, (new((nz, nx, ny, width), dtype=F32, device=device) if fill or width < 8 else None)
 
 
 def project_batch(lors: torch.Tensor, images: torch.Tensor, center, size, *,
