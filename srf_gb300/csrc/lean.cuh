@@ -36,8 +36,10 @@
 // within it skip the reference's range tests (siddon.cu.cc:88-189) and run up to four at a time
 // without a branch between them, so that their instruction chains interleave; other groups run the
 // tests one group at a time. A LOR whose coordinates step more than one voxel per slab (non-square
-// voxels, steep LORs) has no interior. Gathers and reductions are predicated on a non-zero weight (a
-// zero-weight slot of an interior group still has a valid address).
+// voxels, steep LORs) has no interior, nor has one whose first endpoint lies more than kInteriorReach voxels
+// away: its q faces round by 2^-24 of that distance in each of about five operations, a quarter of the margin
+// at 8192 and an offset outside the image from about 1e6 on. Gathers and reductions are predicated on a
+// non-zero weight.
 //
 // Interior groups work on two slabs per lane at a time in packed FP32 (one instruction, two
 // independent roundings, each that of the scalar operation): the loop is bound by instruction issue.
@@ -50,6 +52,7 @@ namespace srf {
 constexpr float kFloorMagic = 12582912.0f;   // 1.5 * 2^23
 constexpr int kFloorBits = 0x4B400000;       // bit pattern of kFloorMagic
 constexpr float kInteriorMargin = 0.01f;     // voxel units
+constexpr float kInteriorReach = 8192.0f;    // voxel units
 
 struct __align__(16) LeanRec {
     float invq, invz, Bz, Z1;     // 1/|q step|, 1/|z step| per slab; z faces: fma(Bz, pp, Z1 or Z2)
@@ -185,7 +188,9 @@ __device__ __forceinline__ LeanRec make_lean(const LorRec &R, const Grid &g, con
     face_interval(R.Az - R.Bz * np2, R.Bz, R.rBz, (float)g.nz, kInteriorMargin, za, zb);
     const float fa = fmaxf(qa, za), fb = fminf(qb, zb);   // faces f in [fa, fb]
     const float il = fmaxf(ceilf(fa), (float)lo), ih = fminf(floorf(fb) - 1.0f, (float)hi);
-    const bool inner = il <= ih && fabsf(R.Bq) <= 1.0f + 1e-5f && fabsf(R.Bz) <= 1.0f + 1e-5f;
+    // (an endpoint far away: the q faces of its LOR round by more than the margin)
+    const bool inner = il <= ih && fabsf(R.Bq) <= 1.0f + 1e-5f && fabsf(R.Bz) <= 1.0f + 1e-5f &&
+                       fmaxf(fabsf(R.p1), fabsf(R.q1)) * E.rdq <= kInteriorReach;
     E.ilo = inner ? (int)il : 1;
     E.ihi = inner ? (int)ih : 0;
     E.plo = (R.flags & F_PROJ) ? max(lo, R.pmlo) : 1;
