@@ -289,6 +289,7 @@ k_emap_columns(EmapCols c, Grid g, View v, View vt, int tiles) {
     const TofParams tp{0, 0, 0};
     const GridK k = make_gridk<false>(g, tp);
     const int nz = g.nz;
+    const double rdx = (double)g.nx / g.sx, dx_dy = (double)g.ny / g.sy / rdx;  // 1 / voxel size, x per y voxel size
     float *s = s_cells + lane;
     for (int r = 0; r < 2 * kWindow; ++r) s[r * 32] = 0.0f;
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
@@ -323,7 +324,19 @@ k_emap_columns(EmapCols c, Grid g, View v, View vt, int tiles) {
         const float ua = bcoord(q1, kq, pp1, p1, dq, nq2, q_one), ub = bcoord(q1, kq, pp2, p1, dq, nq2, q_one);
         const float qq1 = kq >= 0.0f ? ua : ub, qq2 = kq >= 0.0f ? ub : ua;
         const int cq1 = ifloor(qq1), cq2 = ifloor(qq2);
-        const float fq = cq1 != cq2 ? ((float)cq2 - qq1) / (qq2 - qq1) : 1.0f;
+        // The fraction before the crossing, from the lower face in 64 bits; the floors are the reference's. In FP32
+        // its rounding was the image's error: line by line the two orders of a pair round independently, here one
+        // counts twice (40 clinical columns: 1.29e-5 from 64 bits, line by line 1.19e-5, with this 1.5e-6). Once per
+        // slab and column pair: 84.5 ms before, 84.3 ms with it. (The axial coordinate stays in FP32: on
+        // steep lines the reference jumps at voxel faces, and its error does not show beside the fraction's.)
+        float fq = 1.0f;
+        if (cq1 != cq2) {
+            const double u1 = ((double)(xdom ? pa.x : pa.y) - (xdom ? g.cx : g.cy)) * rdx;
+            const double v1 = ((double)(xdom ? pa.y : pa.x) - (xdom ? g.cy : g.cx)) * rdx;
+            const double k64 = ((double)(xdom ? pb.y : pb.x) - (xdom ? pa.y : pa.x)) / ((double)(xdom ? pb.x : pb.y) - (xdom ? pa.x : pa.y));
+            const double lower = (v1 + k64 * ((double)(kq >= 0.0f ? pp1 : pp2) - u1)) * (xdom ? dx_dy : 1.0) + 0.5 * nq;
+            fq = fminf(fmaxf((float)((double)cq2 - lower) * fabsf(dq / kq), 0.0f), 1.0f);
+        }
         const bool okA = act && 0 <= cq1 && cq1 < nq, okB = act && 0 <= cq2 && cq2 < nq && cq1 >= -1;
         if (!__any_sync(0xffffffffu, okA || okB)) continue;
         const float t_lo = __fdiv_rn(__fsub_rn(pp1, p1), pd), t_hi = __fdiv_rn(__fsub_rn(pp2, p1), pd);
