@@ -453,7 +453,7 @@ __device__ __forceinline__ float gather_slots(const float *__restrict__ im, cons
 // views as parameters are as before.
 __device__ __forceinline__ void red_add(float *p, float v) {
 #ifdef __CUDA_ARCH__
-    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
 #else
     atomicAdd(p, v);
 #endif
@@ -465,7 +465,7 @@ __device__ __forceinline__ void red_add(float *p, float v) {
 __device__ __forceinline__ void red_add_where(float w, float *p, float v) {
 #ifdef __CUDA_ARCH__
     asm volatile("{.reg .pred q; setp.neu.f32 q, %2, 0f00000000; @q red.global.add.f32 [%0], %1;}"
-                 ::"l"(__cvta_generic_to_global(p)), "f"(v), "f"(w));
+                 ::"l"(__cvta_generic_to_global(p)), "f"(v), "f"(w) : "memory");
 #else
     if (w != 0.0f) atomicAdd(p, v);
 #endif
