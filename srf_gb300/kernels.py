@@ -53,11 +53,6 @@ def new_xfast(shape: Sequence[int], device) -> torch.Tensor:
     return torch.zeros((nz, ny, nx), dtype=F32, device=device).permute(2, 1, 0)
 
 
-def new_yfast(shape: Sequence[int], device) -> torch.Tensor:
-    nx, ny, nz = shape
-    return torch.zeros((nz, nx, ny), dtype=F32, device=device).permute(1, 2, 0)
-
-
 def _relayout(shape, src: torch.Tensor, src2: Optional[torch.Tensor], dst: torch.Tensor,
               dst2: Optional[torch.Tensor] = None) -> None:
     """dst = src (+ src2), and dst2 the same: (nx, ny, nz) views of any strides, one pass."""
