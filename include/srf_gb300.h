@@ -129,7 +129,8 @@ int srf_projection_adjoint(const float *lors, int64_t n, int32_t lor_stride,
  * gradient of the differentiable projector). Image b starts batch_stride elements after image b-1
  * in each layout given (images and the optional images_t); LOR values / outputs are n_images rows
  * of n at row stride out_stride / values_stride. tof == NULL selects the non-TOF projector. Each
- * LOR is set up and traversed once for all images. */
+ * LOR is set up and traversed once for all images. (The package's batched calls take the interleaved
+ * forms below; these serve images whose interleaved offsets would leave 31 bits.) */
 int srf_projection_batch(const float *lors, int64_t n, int32_t lor_stride, const float *tof,
                          int32_t tof_stride, float tof_bin, float tof_sigma2, float tof_nsigma,
                          int32_t n_images, int64_t batch_stride, const float *images,
@@ -149,7 +150,8 @@ int srf_projection_adjoint_batch(const float *lors, int64_t n, int32_t lor_strid
  * y-dominant LORs' part). Same visits and weights as the forms above, several times fewer memory
  * accesses. srf_interleave fills il (and il_t) from n_images images of any strides, zeros in the
  * unused places; srf_deinterleave writes il (+ il_t) back. Interleaved images are aligned to
- * 4 * width bytes. The adjoint adds to il and il_t. */
+ * 4 * width bytes. The adjoint adds to il and il_t; with il alone a voxel's sum has twice the rms rounding
+ * error. */
 int srf_interleave(const float *images, int64_t batch_stride, const int64_t image_strides[3],
                    int32_t n_images, int32_t width, const int32_t grid[3], float *il, float *il_t,
                    void *stream);
